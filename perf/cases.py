@@ -95,7 +95,8 @@ def draw(rng):
     if kind == "adsorption":
         n = _log_int(rng, 64, 600)
         return dict(kind="run", image=image, n=n, levels=1, steps=rng.randint(60, 200 if n > 250 else 100),
-                    rmin=max(3, n // 100), rmax=max(8, n // 18), porosity=porosity, kn=0.1, sim="adsorption", psi_form=rng.choice([0, 1]))
+                    rmin=max(3, n // 100), rmax=max(8, n // 18), porosity=porosity, kn=0.1, sim="adsorption",
+                    psi_form=rng.choice([0, 1]))
     if kind == "batch":
         sides = [rng.choice([128, 256, 512, 1024]) for _ in range(rng.randint(2, 5))]
         levels = [rng.randint(1, 3 if n == 256 else 2) for n in sides]
