@@ -6,145 +6,15 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 #include "../../../include/mantiis_cnn.h"
+#include "conv_fma.cuh"
 #include "conv_tc.cuh"
 
 namespace
 {
-constexpr int TS = 16;  // pixel tile side
-constexpr int COB = 16; // output channels per block
-constexpr int CIB = 16; // input channels per shared-memory chunk
-
-__device__ __forceinline__ float bf(const uint16_t v) { return __bfloat162float(__ushort_as_bfloat16(v)); }
-
-// y[co] = sum_ci sum_k w[co][ci][k] x[ci](p + offset(k)), offsets (kx - 1, ky - 1)
-// with k = 3 ky + kx.  TRANSPOSE: the data gradient of such a convolution, i.e.
-// the same with w[ci][co][8 - k] (channels swapped, kernel flipped); `cin` and
-// `cout` are this convolution's own input / output channel counts.
-template <bool TRANSPOSE>
-__global__ void __launch_bounds__(256) k_conv3x3(const float *__restrict__ x, const uint16_t *__restrict__ w,
-                                                 const float *__restrict__ b, float *__restrict__ y, int cin,
-                                                 int cout, int h, int wd, int relu)
-{
-    __shared__ float sx[CIB][TS + 2][TS + 2];
-    __shared__ float sw[COB][CIB][9];
-    const int tiles_x = (wd + TS - 1) / TS;
-    const int tx0 = ((int)blockIdx.x % tiles_x) * TS, ty0 = ((int)blockIdx.x / tiles_x) * TS;
-    const int co0 = (int)blockIdx.y * COB;
-    const int n = (int)blockIdx.z;
-    const int lx = threadIdx.x % TS, ly = threadIdx.x / TS;
-    const size_t plane = (size_t)h * wd;
-    float acc[COB];
-#pragma unroll
-    for (int c = 0; c < COB; c++) acc[c] = 0.f;
-    for (int ci0 = 0; ci0 < cin; ci0 += CIB)
-    {
-        for (int i = threadIdx.x; i < CIB * (TS + 2) * (TS + 2); i += blockDim.x)
-        {
-            const int c = i / ((TS + 2) * (TS + 2)), r = i % ((TS + 2) * (TS + 2));
-            const int yy = r / (TS + 2), xx = r % (TS + 2);
-            const int gy = ty0 + yy - 1, gx = tx0 + xx - 1, gc = ci0 + c;
-            float v = 0.f;
-            if (gc < cin && gy >= 0 && gy < h && gx >= 0 && gx < wd)
-                v = x[((size_t)n * cin + gc) * plane + (size_t)gy * wd + gx];
-            sx[c][yy][xx] = v;
-        }
-        for (int i = threadIdx.x; i < COB * CIB * 9; i += blockDim.x)
-        {
-            const int co = i / (CIB * 9), r = i % (CIB * 9), c = r / 9, k = r % 9;
-            const int gco = co0 + co, gci = ci0 + c;
-            float v = 0.f;
-            if (gco < cout && gci < cin)
-                v = TRANSPOSE ? bf(w[((size_t)gci * cout + gco) * 9 + (8 - k)]) : bf(w[((size_t)gco * cin + gci) * 9 + k]);
-            sw[co][c][k] = v;
-        }
-        __syncthreads();
-        const int cmax = min(CIB, cin - ci0);
-        for (int c = 0; c < cmax; c++)
-        {
-#pragma unroll
-            for (int k = 0; k < 9; k++)
-            {
-                const float xv = sx[c][ly + k / 3][lx + k % 3];
-#pragma unroll
-                for (int co = 0; co < COB; co++) acc[co] = fmaf(sw[co][c][k], xv, acc[co]);
-            }
-        }
-        __syncthreads();
-    }
-    const int px = tx0 + lx, py = ty0 + ly;
-    if (px >= wd || py >= h) return;
-#pragma unroll
-    for (int co = 0; co < COB; co++)
-    {
-        const int gco = co0 + co;
-        if (gco >= cout) break;
-        float v = acc[co] + (b ? b[gco] : 0.f);
-        if (relu) v = fmaxf(v, 0.f);
-        y[((size_t)n * cout + gco) * plane + (size_t)py * wd + px] = v;
-    }
-}
-
-// dw[co][ci][k] += sum_pixels dy[co](p) x[ci](p + offset(k)); db[co] += sum dy[co]
-__global__ void __launch_bounds__(256) k_conv3x3_bw(const float *__restrict__ x, const float *__restrict__ dy,
-                                                    float *__restrict__ dw, float *__restrict__ db, int cin, int cout,
-                                                    int h, int wd)
-{
-    __shared__ float sdy[COB][TS][TS];
-    __shared__ float sx[CIB][TS + 2][TS + 2];
-    const int tiles_x = (wd + TS - 1) / TS;
-    const int tx0 = ((int)blockIdx.x % tiles_x) * TS, ty0 = ((int)blockIdx.x / tiles_x) * TS;
-    const int nci = (cin + CIB - 1) / CIB;
-    const int co0 = ((int)blockIdx.y / nci) * COB, ci0 = ((int)blockIdx.y % nci) * CIB;
-    const int n = (int)blockIdx.z;
-    const size_t plane = (size_t)h * wd;
-    for (int i = threadIdx.x; i < COB * TS * TS; i += blockDim.x)
-    {
-        const int c = i / (TS * TS), r = i % (TS * TS), yy = r / TS, xx = r % TS;
-        const int gy = ty0 + yy, gx = tx0 + xx, gc = co0 + c;
-        float v = 0.f;
-        if (gc < cout && gy < h && gx < wd) v = dy[((size_t)n * cout + gc) * plane + (size_t)gy * wd + gx];
-        sdy[c][yy][xx] = v;
-    }
-    for (int i = threadIdx.x; i < CIB * (TS + 2) * (TS + 2); i += blockDim.x)
-    {
-        const int c = i / ((TS + 2) * (TS + 2)), r = i % ((TS + 2) * (TS + 2));
-        const int yy = r / (TS + 2), xx = r % (TS + 2);
-        const int gy = ty0 + yy - 1, gx = tx0 + xx - 1, gc = ci0 + c;
-        float v = 0.f;
-        if (gc < cin && gy >= 0 && gy < h && gx >= 0 && gx < wd)
-            v = x[((size_t)n * cin + gc) * plane + (size_t)gy * wd + gx];
-        sx[c][yy][xx] = v;
-    }
-    __syncthreads();
-    const int co = threadIdx.x / CIB, ci = threadIdx.x % CIB;
-    float acc[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[k] = 0.f;
-    for (int yy = 0; yy < TS; yy++)
-        for (int xx = 0; xx < TS; xx++)
-        {
-            const float g = sdy[co][yy][xx];
-#pragma unroll
-            for (int k = 0; k < 9; k++) acc[k] = fmaf(g, sx[ci][yy + k / 3][xx + k % 3], acc[k]);
-        }
-    const int gco = co0 + co, gci = ci0 + ci;
-    if (gco < cout && gci < cin)
-    {
-#pragma unroll
-        for (int k = 0; k < 9; k++) atomicAdd(&dw[((size_t)gco * cin + gci) * 9 + k], acc[k]);
-    }
-    if (db && ci0 == 0 && (int)threadIdx.x < COB && co0 + (int)threadIdx.x < cout)
-    {
-        float s = 0.f;
-        for (int yy = 0; yy < TS; yy++)
-            for (int xx = 0; xx < TS; xx++) s += sdy[threadIdx.x][yy][xx];
-        atomicAdd(&db[co0 + threadIdx.x], s);
-    }
-}
-
 __global__ void k_relu_bw(float *dy, const float *y, int64_t count)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -291,9 +161,92 @@ int tc_ntile(int pixel_ctas, int cout)
     return nt;
 }
 
-dim3 conv_grid(int h, int wd, int groups, int n)
+int sm_count()
 {
-    return dim3((unsigned)(((wd + TS - 1) / TS) * ((h + TS - 1) / TS)), (unsigned)groups, (unsigned)n);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// raises a kernel's dynamic shared memory limit, once per device
+cudaError_t allow_smem(const void *kernel, size_t bytes, std::atomic<uint64_t> &done)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    const cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (r == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return r;
+}
+
+template <typename T, bool TRANSPOSE>
+int launch_conv(const float *x, const uint16_t *w, const float *b, float *y, int n, int cin, int cout, int h, int wd,
+                int relu, cudaStream_t st)
+{
+    static std::atomic<uint64_t> ready{0};
+    const auto kernel = cnn_fma::k_conv3x3_fma<T, TRANSPOSE>;
+    const cudaError_t e = allow_smem((const void *)kernel, T::kSmem, ready);
+    if (e != cudaSuccess) return -(int)e;
+    const dim3 grid((unsigned)(((wd + T::TW - 1) / T::TW) * ((h + T::TH - 1) / T::TH)),
+                    (unsigned)((cout + T::CO - 1) / T::CO), (unsigned)n);
+    kernel<<<grid, T::kThreads, T::kSmem, st>>>(x, w, b, y, cin, cout, h, wd, relu);
+    return done();
+}
+
+// Register tiles of the FP32 convolutions, largest first: 512 pixels x 32
+// channels (64 sums a thread), 256 x 32 (32), 128 x 32 (16), 64 x 16 (8), and
+// 256 x 8 for layers of few output channels.
+using ConvA = cnn_fma::ConvTile<32, 16, 2, 4, 8, 8>;
+using ConvB = cnn_fma::ConvTile<32, 8, 1, 4, 8, 8>;
+using ConvC = cnn_fma::ConvTile<16, 8, 1, 8, 4, 8>;
+using ConvD = cnn_fma::ConvTile<8, 8, 1, 8, 2, 16>;
+using ConvE = cnn_fma::ConvTile<32, 8, 1, 2, 4, 8>;
+
+// Time of a tile on a layer in units of one FMA per sum: rounds of blocks over
+// the SMs x sums per block x the tile's cost per FMA, which comes from sweeps of
+// every tile over the network's layers (a full GPU of A runs at 45-51 TFLOP/s, B
+// 43-50, C 29-34, D 20; layers that fill the GPU with A fall to 5-10 TFLOP/s at
+// 16^2 and 8^2 pixels, where C and D reach 25 and 12.5)
+template <typename T> double conv_cost(int n, int cout, int h, int wd, int sms, double per_fma)
+{
+    const int64_t blocks = (int64_t)((wd + T::TW - 1) / T::TW) * ((h + T::TH - 1) / T::TH) * ((cout + T::CO - 1) / T::CO) * n;
+    return (double)((blocks + sms - 1) / sms) * T::ACC * T::kThreads * per_fma;
+}
+
+template <bool TRANSPOSE>
+int conv(const float *x, const uint16_t *w, const float *b, float *y, int n, int cin, int cout, int h, int wd, int relu,
+         cudaStream_t st)
+{
+    const int sms = sm_count();
+    const double cost[5] = {conv_cost<ConvA>(n, cout, h, wd, sms, 1.0), conv_cost<ConvB>(n, cout, h, wd, sms, 1.06),
+                            conv_cost<ConvC>(n, cout, h, wd, sms, 1.5), conv_cost<ConvD>(n, cout, h, wd, sms, 2.3),
+                            conv_cost<ConvE>(n, cout, h, wd, sms, 1.5)};
+    switch ((int)(std::min_element(cost, cost + 5) - cost))
+    {
+    case 0: return launch_conv<ConvA, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
+    case 1: return launch_conv<ConvB, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
+    case 2: return launch_conv<ConvC, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
+    case 3: return launch_conv<ConvD, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
+    default: return launch_conv<ConvE, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
+    }
+}
+
+template <typename T>
+int launch_wgrad(const float *x, const float *dy, float *dw, float *db, int n, int cin, int cout, int h, int wd,
+                 cudaStream_t st)
+{
+    static std::atomic<uint64_t> ready{0};
+    const auto kernel = cnn_fma::k_conv3x3_wgrad_fma<T>;
+    const cudaError_t e = allow_smem((const void *)kernel, T::kSmem, ready);
+    if (e != cudaSuccess) return -(int)e;
+    const int64_t groups = (int64_t)((cout + T::CO - 1) / T::CO) * ((cin + T::LCI - 1) / T::LCI);
+    const int64_t tiles = (int64_t)((wd + T::TW - 1) / T::TW) * ((h + T::TH - 1) / T::TH) * n;
+    // two blocks per SM share a channel group's pixel tiles
+    const int64_t split = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(tiles, 65535), 2 * sm_count() / groups));
+    kernel<<<dim3((unsigned)groups, (unsigned)split), cnn_fma::kThreads, T::kSmem, st>>>(x, dy, dw, db, n, cin, cout, h, wd);
+    return done();
 }
 } // namespace
 
@@ -303,9 +256,7 @@ int cnn_conv3x3_forward(const float *x, const uint16_t *w, const float *b, float
                         int wd, int relu, void *stream)
 {
     if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0) return -1;
-    k_conv3x3<false><<<conv_grid(h, wd, (cout + COB - 1) / COB, n), 256, 0, (cudaStream_t)stream>>>(x, w, b, y, cin,
-                                                                                                   cout, h, wd, relu);
-    return done();
+    return conv<false>(x, w, b, y, n, cin, cout, h, wd, relu, (cudaStream_t)stream);
 }
 
 int cnn_conv3x3_backward_data(const float *dy, const uint16_t *w, float *dx, int n, int cin, int cout, int h, int wd,
@@ -313,9 +264,7 @@ int cnn_conv3x3_backward_data(const float *dy, const uint16_t *w, float *dx, int
 {
     if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0) return -1;
     // a convolution from the cout gradient channels to the cin input channels
-    k_conv3x3<true><<<conv_grid(h, wd, (cin + COB - 1) / COB, n), 256, 0, (cudaStream_t)stream>>>(dy, w, nullptr, dx,
-                                                                                                  cout, cin, h, wd, 0);
-    return done();
+    return conv<true>(dy, w, nullptr, dx, n, cout, cin, h, wd, 0, (cudaStream_t)stream);
 }
 
 int cnn_conv3x3_forward_tc(const float *x, const uint16_t *w, const float *b, float *y, int n, int cin, int cout,
@@ -383,9 +332,16 @@ int cnn_conv3x3_backward_weight(const float *x, const float *dy, float *dw, floa
                                 int wd, void *stream)
 {
     if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0) return -1;
-    const int groups = ((cout + COB - 1) / COB) * ((cin + CIB - 1) / CIB);
-    k_conv3x3_bw<<<conv_grid(h, wd, groups, n), 256, 0, (cudaStream_t)stream>>>(x, dy, dw, db, cin, cout, h, wd);
-    return done();
+    const cudaStream_t st = (cudaStream_t)stream;
+    // 16 x 8 pixel tiles, 8 x 8 where the image is no wider; with few output
+    // (input) channels the warps (lanes) share the pixels instead of channels
+    using namespace cnn_fma;
+    if (cout <= 8)
+        return wd > 8 ? launch_wgrad<WgradTile<16, 8, 1, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st)
+                      : launch_wgrad<WgradTile<8, 8, 1, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st);
+    if (cin <= 4) return launch_wgrad<WgradTile<16, 8, 8, 4>>(x, dy, dw, db, n, cin, cout, h, wd, st);
+    return wd > 8 ? launch_wgrad<WgradTile<16, 8, 8, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st)
+                  : launch_wgrad<WgradTile<8, 8, 8, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st);
 }
 
 int cnn_relu_backward(float *dy, const float *y, int64_t count, void *stream)

@@ -32,10 +32,10 @@ _cnn = None
 # True: the convolutions' forward and data gradient run as the tcgen05 implicit
 # GEMMs (cnn_conv3x3_*_tc).  Their operand staging (the threads gather the patch
 # matrix and split it into two BF16 parts in shared memory, one stage) bounds
-# them at 6-12 TFLOP/s, below the CUDA-core kernels' 10-14.5 at this network's
-# layer sizes (8 x 32..256 channels, 16^2..128^2 pixels; bench.py --conv), so
-# those stay the default; both agree with FP64 to within 6e-6 of the largest
-# output.
+# them at 6-12 TFLOP/s, below the register-tiled FP32 kernels' 25-51 at this
+# network's layer sizes (8 x 32..256 channels, 16^2..128^2 pixels; bench.py
+# --conv), and two BF16 parts hold 16 bits of an activation, not 24 (2-6e-6 of
+# the largest output against 0.1-2e-6), so those stay the default.
 TENSOR_CORES = False
 
 _P = C.c_void_p
