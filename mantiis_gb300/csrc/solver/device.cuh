@@ -206,27 +206,35 @@ __device__ __forceinline__ void inv_moments(const float m[9], float v[9])
     v[8] = ad + jx - jy - m[8] * 0.25f;
 }
 
-// relaxation rates diag(1, 1/1.1, 1/1.2, 1/tau_d, 1/tau_q, 1/tau_d, 1/tau_q, 1/tau_s, 1/tau_s)
-__device__ __forceinline__ void rates(float tau_s, float tau_d, float s[9])
+// The cell-dependent rates of diag(1, 1/1.1, 1/1.2, 1/tau_d, 1/tau_q, 1/tau_d, 1/tau_q, 1/tau_s, 1/tau_s)
+struct MrtRates
+{
+    float d, q, s; // 1/tau_d, 1/tau_q, 1/tau_s
+};
+__device__ __forceinline__ MrtRates mrt_rates(float tau_s, float tau_d)
 {
     const float t = 2.0f * tau_s - 1.0f;
     const float tau_q = 0.5f + (3.0f + 3.14159265358979f * t * t * 0.9f) / (8.0f * t);
+    return {1.0f / tau_d, 1.0f / tau_q, 1.0f / tau_s};
+}
+__device__ __forceinline__ void rates(const MrtRates &r, float s[9])
+{
     s[0] = 1.0f;
     s[1] = 1.0f / 1.1f;
     s[2] = 1.0f / 1.2f;
-    s[3] = s[5] = 1.0f / tau_d;
-    s[4] = s[6] = 1.0f / tau_q;
-    s[7] = s[8] = 1.0f / tau_s;
+    s[3] = s[5] = r.d;
+    s[4] = s[6] = r.q;
+    s[7] = s[8] = r.s;
 }
 
 // Plain MRT (include/coreLB.hpp:694-742): f* = f - M^-1 R M (f - f_eq)
-__device__ __forceinline__ void collide_mrt(const float df[9], const float feq[9], float tau_s, float tau_d, float out[9])
+__device__ __forceinline__ void collide_mrt(const float df[9], const float feq[9], const MrtRates &r, float out[9])
 {
     float fn[9], m[9], s[9], dv[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) fn[q] = df[q] - feq[q];
     moments(fn, m);
-    rates(tau_s, tau_d, s);
+    rates(r, s);
 #pragma unroll
     for (int k = 0; k < 9; k++) m[k] *= s[k];
     inv_moments(m, dv);
@@ -237,7 +245,7 @@ __device__ __forceinline__ void collide_mrt(const float df[9], const float feq[9
 // Guo-type MRT source term (include/coreLB.hpp:568-630): f += M^-1 (I - R/2) M S,
 // S_q = w_q [c.F / cs^2 + (u F) : (c c - cs^2 I) / cs^4] with the reference's
 // pairing of the mixed terms (uF[2] with c_x c_y, uF[1] with c_y c_x).
-__device__ __forceinline__ void add_source(float out[9], float ux, float uy, float Fx, float Fy, float tau_s, float tau_d)
+__device__ __forceinline__ void add_source(float out[9], float ux, float uy, float Fx, float Fy, const MrtRates &r)
 {
     float S[9], m[9], s[9], dv[9];
     const float uFxx = ux * Fx, uFxy = ux * Fy, uFyx = uy * Fx, uFyy = uy * Fy;
@@ -250,7 +258,7 @@ __device__ __forceinline__ void add_source(float out[9], float ux, float uy, flo
         S[q] = wq(q) * (cF * 3.0f + cc * 9.0f);
     }
     moments(S, m);
-    rates(tau_s, tau_d, s);
+    rates(r, s);
 #pragma unroll
     for (int k = 0; k < 9; k++) m[k] *= (1.0f - 0.5f * s[k]);
     inv_moments(m, dv);

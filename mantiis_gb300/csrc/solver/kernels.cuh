@@ -136,7 +136,7 @@ __device__ __forceinline__ void step_cell(const LevelView &L, const Common &C, c
     float feq[9], fs[9];
     equilibrium(edrho, erho, eux, euy, feq);
     if (C.collision == COLL_RMRT) collide_rmrt(df, feq, edrho, erho, eux, euy, omega, fs);
-    else if (C.collision == COLL_MRT) collide_mrt(df, feq, 1.0f / omega, L.tau2 ? L.tau2[s] : 1.0f, fs);
+    else if (C.collision == COLL_MRT) collide_mrt(df, feq, mrt_rates(1.0f / omega, L.tau2 ? L.tau2[s] : 1.0f), fs);
     else
     {
         const float inv_tau = 1.0f; // 1 / tau_SRT, tau_SRT = 1 (include/globalParameters.hpp:140)
@@ -643,24 +643,16 @@ template <int P> __global__ void __launch_bounds__(128) k_ads_psi_special(LevelV
 // the same body with the regularized MRT, SRBB walls, no inlet / outlet and the
 // velocity residual (C.collision, C.wall, C.inlet_outlet; o.diff accumulates
 // sum |u| for both terms, as its |u| of the previous step is never stored).
-// psi[r][c]: the pseudopotential at (x + c - 1, y + r - 1); SPEC: the cell may
-// be special (its record applies), else it is a plain cell
-template <int P, bool SPEC>
-__device__ __forceinline__ void ads_cell(const LevelView &L, const Common &C, const StepOpt &o, int x, int y,
-                                         const float psi[3][3], double &r_diff, double &r_norm)
+// psi[r][c]: the pseudopotential at (x + c - 1, y + r - 1); df: the cell's
+// populations, mr its relaxation rates (omega: 1/tau_s for the regularized
+// MRT); special: its record applies.
+template <int P>
+__device__ __forceinline__ void ads_update(const LevelView &L, const Common &C, const StepOpt &o, int x, int y,
+                                           const float df[9], float omega, const MrtRates &mr, bool special,
+                                           const SpecialRec &rec, const float psi[3][3], double &r_diff, double &r_norm,
+                                           bool interior = false)
 {
     const int64_t s = site_of(L, x, y);
-    float df[9];
-    bool special = false;
-    SpecialRec rec;
-    float omega;
-    if (SPEC) omega = load_cell<P>(L, C, x, y, o.direct, o.first_sub, df, special, rec);
-    else
-    {
-        if (o.direct) load_raw<0>(L, x, y, df);
-        else load_raw<P>(L, x, y, df);
-        omega = L.omega[s];
-    }
     const uint32_t out = special ? ((rec.m1 >> 21) & 0x1FFu) : 0x1FFu;
     const uint32_t wall = special ? ((rec.m0 >> 18) & 0x1FFu) : 0u;
     // sum over the streaming links of w_f psi(x + c) c, formed from psi differences
@@ -711,10 +703,9 @@ __device__ __forceinline__ void ads_cell(const LevelView &L, const Common &C, co
     }
     float feq[9], fs[9];
     equilibrium(drho, rho, ux, uy, feq);
-    const float tau_s = 1.0f / omega, tau_d = L.tau2[s];
     if (C.collision == COLL_RMRT) collide_rmrt(df, feq, drho, rho, ux, uy, omega, fs);
-    else collide_mrt(df, feq, tau_s, tau_d, fs);
-    add_source(fs, ux, uy, Fx, Fy, tau_s, tau_d);
+    else collide_mrt(df, feq, mr, fs);
+    add_source(fs, ux, uy, Fx, Fy, mr);
     if (special && (rec.m1 & 0x1FFu))
     {
         const uint32_t quirk = rec.m1 & 0x1FFu;
@@ -724,7 +715,28 @@ __device__ __forceinline__ void ads_cell(const LevelView &L, const Common &C, co
         for (int q = 0; q < 9; q++)
             if ((quirk >> q) & 1u) side_now[rec.quirk_base + qi++] = fs[q];
     }
-    store_post<P>(L, x, y, fs);
+    store_post<P>(L, x, y, fs, interior);
+}
+
+// The same of a cell whose populations are loaded here.  SPEC: the cell may be
+// special, else it is a plain cell.
+template <int P, bool SPEC>
+__device__ __forceinline__ void ads_cell(const LevelView &L, const Common &C, const StepOpt &o, int x, int y,
+                                         const float psi[3][3], double &r_diff, double &r_norm)
+{
+    const int64_t s = site_of(L, x, y);
+    float df[9];
+    bool special = false;
+    SpecialRec rec;
+    float omega;
+    if (SPEC) omega = load_cell<P>(L, C, x, y, o.direct, o.first_sub, df, special, rec);
+    else
+    {
+        if (o.direct) load_raw<0>(L, x, y, df);
+        else load_raw<P>(L, x, y, df);
+        omega = L.omega[s];
+    }
+    ads_update<P>(L, C, o, x, y, df, omega, mrt_rates(1.0f / omega, L.tau2[s]), special, rec, psi, r_diff, r_norm);
 }
 
 // Pass 2 over the plain cells of active 32x8 tile t: one block.  The
@@ -1226,33 +1238,78 @@ __global__ void __launch_bounds__(kPersistThreads, MINB) k_step_persistent(const
 
 // ---- the adsorption step as one cooperative launch over many steps.  Each
 // step is the two passes of k_ads_psi / k_ads_psi_special and k_ads_step /
-// k_ads_step_special over the same units (32x8 tiles, then runs of 256 special
-// records), walked by a grid that is resident as a whole (cooperative launch);
-// a grid barrier closes each pass.  The per-cell arithmetic is the same code,
-// so the states are bit-identical to the launch-per-pass engine.
+// k_ads_step_special, each closed by a grid barrier; the per-cell arithmetic is
+// the same code, so the states are bit-identical to the launch-per-pass engine.
+//
+// What bounds a step at these sizes (156 k cells: 1 k per SM) is latency: two
+// grid barriers, a round trip to L2 for the populations and one for the
+// neighbours' pseudopotentials, then the instructions of pass 2 (about 700 per
+// warp of cells).  So one block per SM (fewest arrivals at a barrier) owns the
+// same cells in every step, an equal share of the plain cells and of the special
+// records, a warp at a time; it keeps what only it reads in shared memory:
+// the populations between the two passes, the relaxation rates, the density of
+// the previous step.  Populations are then read once a step, the density and
+// the outputs leave for memory in the last step of the launch only.  Measured on
+// a GB300, us per step: 512^2 image (156 k cells) 9.2, 190^2 6.9, 64^2 5.8 (a
+// barrier alone is 1.3); with tiles dealt to 456 blocks that read the populations
+// in both passes 24.4, 13.9 and 11.1.
 struct AdsPersist
 {
     LevelView L;
     Common C;
+    const int32_t *plain_xy; // plain cells, row-major: x | y << 16
     int64_t spec_begin;
-    int spec_count, ntiles;
+    int nplain, spec_count;
+    int slots;              // cells' warps whose data fits a block's shared memory
+    int rec_slots;          // of these, warps of special cells (their records come first)
     int nsteps, parity0, direct0;
     int slot0, ring;        // residual of step k in slot (slot0 + k) mod ring
-    int psi_diff, step_diff; // the residual terms of pass 1 (density change) / pass 2 (|u|)
+    int psi_diff;           // accumulate the residual of pass 1 (density change)
     unsigned int *bar;      // arrivals at the grid barriers; zero at launch
 };
+
+// shared memory of one warp of cells: this many floats per lane
+constexpr int kAdsFields = 15;
+enum AdsField
+{
+    AF_F = 0,    // 9 populations, as the cell collides
+    AF_RATE = 9, // relaxation rates 1/tau_d, 1/tau_q, 1/tau_s
+    AF_PSI = 12, // the cell's pseudopotential
+    AF_RHO = 13, // its density in the previous step
+    AF_XY = 14,  // x | y << 16 of a plain cell, negative past the end
+};
+constexpr size_t kAdsSlotBytes = (size_t)kAdsFields * 32 * 4;
+constexpr size_t kAdsRecBytes = (size_t)32 * sizeof(SpecialRec); // records of one warp of special cells
+// Most threads of a block: blocks of one round of warps take the kernel of up to
+// 512 threads (128 registers, nothing spilled), the others that of up to 640 (96)
+constexpr int kAdsSmall = 512, kAdsLarge = 640;
 
 // Grid barrier `target` = (barriers passed) x gridDim.x: every block adds one
 // arrival with release semantics after its block barrier, then waits (bounded)
 // for all of them; a wait that runs out sets the error word and the block stops.
-__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int target, unsigned int *err)
+// rmax: if not null, the block's maximum of the residual terms (non-negative
+// floats by their bit patterns), which goes to dst and is cleared.
+__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int target, unsigned int *err,
+                                             unsigned int *rmax, double *dst)
 {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0)
     {
+        if (rmax && *rmax)
+        {
+            atomicMax(reinterpret_cast<unsigned long long *>(dst),
+                      (unsigned long long)__double_as_longlong((double)__uint_as_float(*rmax)));
+            *rmax = 0u;
+        }
         add_release(bar, 1u);
-        const bool ok = wait_counter(bar, target);
+        bool ok = false;
+        for (uint32_t i = 0; i < kDepPolls && !ok; i++)
+        {
+            unsigned int v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            ok = v >= target;
+        }
         if (!ok) atomicOr(err, kErrDepTimeout);
         s_ok = ok ? 1 : 0;
     }
@@ -1260,58 +1317,294 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int tar
     return s_ok != 0;
 }
 
-constexpr int kAdsRecords = 256; // special records per unit of k_ads_persistent
-
-__global__ void __launch_bounds__(256) k_ads_persistent(const __grid_constant__ AdsPersist A)
+// the neighbours' pseudopotentials around (x, y); the centre is the caller's
+__device__ __forceinline__ void load_psi(const LevelView &L, int x, int y, bool interior, float psi[3][3])
 {
-    const int units = A.ntiles + (A.spec_count + kAdsRecords - 1) / kAdsRecords;
+    if (interior)
+    {
+        const float *p = L.psi + site_of(L, x, y);
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                if (r != 1 || c != 1) psi[r][c] = p[(r - 1) * (int64_t)L.pitch + c - 1];
+    }
+    else
+    {
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                if (r != 1 || c != 1) psi[r][c] = L.psi[site_of(L, wrapx(x + c - 1, L.W), wrapx(y + r - 1, L.H))];
+    }
+}
+
+// The block's cells: special records [s0, s1) in ws warps, plain cells [p0, p1)
+// in wp warps.  Slot k of the shared memory belongs to warp-of-cells k.  The
+// special ones go to the block's warps from the first on; a special cell takes
+// about as long as two plain ones, so plain ones go to the warps after those
+// where there are enough (first plain warp of this warp: pj0, then every pstep).
+struct AdsShare
+{
+    int s0, s1, p0, p1, ws, wp, pj0, pstep;
+    uint4 *recs; // special records of the first rec_slots warps, as [warp][half][lane]
+};
+
+// One warp of cells of the block as a lane sees it: the cell, and its data in
+// shared memory (m; null where FITS is false and the slots ran out).
+template <bool FITS> struct AdsCell
+{
+    const LevelView &L;
+    float *m;
+    int x, y;
+    int64_t s;
+    __device__ __forceinline__ AdsCell(const AdsPersist &A, float *sm, int u, int xy)
+        : L(A.L), m(FITS || u < A.slots ? sm + (size_t)u * kAdsFields * 32 + (threadIdx.x & 31) : nullptr),
+          x(xy & 0xFFFF), y(xy >> 16), s(site_of(A.L, x, y))
+    {
+    }
+    __device__ __forceinline__ bool held() const { return FITS || m != nullptr; }
+    __device__ __forceinline__ bool interior() const { return x > 0 && x + 1 < L.W && y > 0 && y + 1 < L.H; }
+    __device__ __forceinline__ float old_density() const { return held() ? m[AF_RHO * 32] : L.rho_prev[s]; }
+    __device__ __forceinline__ MrtRates rates(float omega) const
+    {
+        if (held()) return MrtRates{m[AF_RATE * 32], m[(AF_RATE + 1) * 32], m[(AF_RATE + 2) * 32]};
+        return mrt_rates(1.0f / omega, L.tau2[s]);
+    }
+    // pass 1 with the populations df: pseudopotential, density change returned
+    __device__ __forceinline__ float density(const Common &C, const float df[9], float old, bool last)
+    {
+        float drho = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 9; q++) drho += df[q];
+        const float rho = C.rho0 + drho;
+        const float psi = pseudo_potential((float)C.psi_form, C.psi_rho0, C.eos_a, C.eos_b, C.eos_T, C.g_ff, rho);
+        L.psi[s] = psi;
+        if (!held() || last) L.rho_prev[s] = rho;
+        if (held())
+        {
+#pragma unroll
+            for (int q = 0; q < 9; q++) m[(AF_F + q) * 32] = df[q];
+            m[AF_PSI * 32] = psi;
+            m[AF_RHO * 32] = rho;
+        }
+        return fabsf(rho - old) / old;
+    }
+    __device__ __forceinline__ void populations(float df[9]) const
+    {
+#pragma unroll
+        for (int q = 0; q < 9; q++) df[q] = m[(AF_F + q) * 32];
+    }
+};
+
+// record of lane `lane` of special warp u (record i of the level)
+__device__ __forceinline__ SpecialRec ads_record(const AdsPersist &A, const AdsShare &B, int u, int i, int lane)
+{
+    if (u >= A.rec_slots) return A.C.specials[A.spec_begin + i];
+    union
+    {
+        SpecialRec rec;
+        uint4 v[2];
+    } t;
+    static_assert(sizeof(SpecialRec) == 2 * sizeof(uint4), "record size");
+    t.v[0] = B.recs[(u * 2) * 32 + lane];
+    t.v[1] = B.recs[(u * 2 + 1) * 32 + lane];
+    return t.rec;
+}
+
+// x | y << 16 of this lane's cell in plain warp j, negative past the share
+template <bool FITS> __device__ __forceinline__ int ads_plain_xy(const AdsPersist &A, const AdsShare &B, const float *sm, int j)
+{
+    const int u = B.ws + j, lane = threadIdx.x & 31;
+    if (FITS || u < A.slots) return __float_as_int(sm[((size_t)u * kAdsFields + AF_XY) * 32 + lane]);
+    const int i = B.p0 + j * 32 + lane;
+    return i < B.p1 ? __ldg(&A.plain_xy[i]) : -1;
+}
+
+// fills the block's shared memory: records, cells, relaxation rates and
+// previous densities
+__device__ __forceinline__ void ads_fill(const AdsPersist &A, const AdsShare &B, float *sm)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int u = warp; u < B.ws + B.wp && u < A.slots; u += nw)
+    {
+        float *m = sm + (size_t)u * kAdsFields * 32 + lane;
+        int xy = -1;
+        float omega = 0.0f;
+        if (u < B.ws)
+        {
+            const int i = B.s0 + u * 32 + lane;
+            if (i < B.s1)
+            {
+                const uint4 *r = reinterpret_cast<const uint4 *>(A.C.specials + A.spec_begin + i);
+                const uint4 r0 = r[0], r1 = r[1];
+                if (u < A.rec_slots)
+                {
+                    B.recs[(u * 2) * 32 + lane] = r0;
+                    B.recs[(u * 2 + 1) * 32 + lane] = r1;
+                }
+                xy = (int)r1.z;
+                omega = __uint_as_float(r1.w);
+            }
+        }
+        else
+        {
+            const int i = B.p0 + (u - B.ws) * 32 + lane;
+            if (i < B.p1) xy = __ldg(&A.plain_xy[i]);
+            if (xy >= 0) omega = A.L.omega[site_of(A.L, xy & 0xFFFF, xy >> 16)];
+        }
+        m[AF_XY * 32] = __int_as_float(xy);
+        if (xy < 0) continue;
+        const int64_t s = site_of(A.L, xy & 0xFFFF, xy >> 16);
+        const MrtRates r = mrt_rates(1.0f / omega, A.L.tau2[s]);
+        m[AF_RATE * 32] = r.d;
+        m[(AF_RATE + 1) * 32] = r.q;
+        m[(AF_RATE + 2) * 32] = r.s;
+        m[AF_RHO * 32] = A.L.rho_prev[s];
+    }
+}
+
+template <int P, bool FITS>
+__device__ __forceinline__ float ads_pass1(const AdsPersist &A, const AdsShare &B, float *sm, bool direct, bool last)
+{
+    const LevelView &L = A.L;
+    const Common &C = A.C;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    float rmax = 0.0f;
+#pragma unroll 1
+    for (int u = warp; u < B.ws; u += nw)
+    {
+        const int i = B.s0 + u * 32 + lane;
+        if (i >= B.s1) continue;
+        const SpecialRec rec = ads_record(A, B, u, i, lane);
+        AdsCell<FITS> c(A, sm, u, rec.xy);
+        float df[9];
+        const float old = c.old_density();
+        if (direct) load_raw<0>(L, c.x, c.y, df);
+        else load_special<P>(L, C, rec, c.x, c.y, df);
+        rmax = fmaxf(rmax, c.density(C, df, old, last));
+    }
+    // plain cells, two warps of cells at a time: both populations in flight (a
+    // direct state has parity 0: own slots)
+#pragma unroll 1
+    for (int j0 = B.pj0; j0 < B.wp; j0 += 2 * B.pstep)
+    {
+        float df[2][9];
+        int xy[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+        {
+            xy[k] = j0 + k * B.pstep < B.wp ? ads_plain_xy<FITS>(A, B, sm, j0 + k * B.pstep) : -1;
+            if (xy[k] < 0) continue;
+            const AdsCell<FITS> c(A, sm, B.ws + j0 + k * B.pstep, xy[k]);
+            load_raw_ro<P, false>(L, c.x, c.y, df[k], c.interior());
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+        {
+            if (xy[k] < 0) continue;
+            AdsCell<FITS> c(A, sm, B.ws + j0 + k * B.pstep, xy[k]);
+            rmax = fmaxf(rmax, c.density(C, df[k], c.old_density(), last));
+        }
+    }
+    return rmax;
+}
+
+template <int P, bool FITS>
+__device__ __forceinline__ void ads_pass2(const AdsPersist &A, const AdsShare &B, float *sm, const StepOpt &o, bool direct)
+{
+    const LevelView &L = A.L;
+    const Common &C = A.C;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double none0 = 0.0, none1 = 0.0;
+#pragma unroll 1
+    for (int u = warp; u < B.ws; u += nw)
+    {
+        const int i = B.s0 + u * 32 + lane;
+        if (i >= B.s1) continue;
+        const SpecialRec rec = ads_record(A, B, u, i, lane);
+        const AdsCell<FITS> c(A, sm, u, rec.xy);
+        float psi[3][3], df[9];
+        load_psi(L, c.x, c.y, c.interior(), psi);
+        psi[1][1] = c.held() ? c.m[AF_PSI * 32] : L.psi[c.s];
+        if (c.held()) c.populations(df);
+        else if (direct) load_raw<0>(L, c.x, c.y, df);
+        else load_special<P>(L, C, rec, c.x, c.y, df);
+        ads_update<P>(L, C, o, c.x, c.y, df, rec.omega, c.rates(rec.omega), true, rec, psi, none0, none1);
+    }
+#pragma unroll 1
+    for (int j = B.pj0; j < B.wp; j += B.pstep)
+    {
+        const int xy = ads_plain_xy<FITS>(A, B, sm, j);
+        if (xy < 0) continue;
+        const AdsCell<FITS> c(A, sm, B.ws + j, xy);
+        float psi[3][3], df[9], omega = 0.0f;
+        load_psi(L, c.x, c.y, c.interior(), psi);
+        psi[1][1] = c.held() ? c.m[AF_PSI * 32] : L.psi[c.s];
+        if (c.held()) c.populations(df);
+        else
+        {
+            load_raw_ro<P, false>(L, c.x, c.y, df, c.interior());
+            omega = L.omega[c.s];
+        }
+        const SpecialRec none{};
+        ads_update<P>(L, C, o, c.x, c.y, df, omega, c.rates(omega), false, none, psi, none0, none1, c.interior());
+    }
+}
+
+template <int THREADS, bool FITS>
+__global__ void __launch_bounds__(THREADS, 1) k_ads_persistent(const __grid_constant__ AdsPersist A)
+{
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ unsigned int s_rmax;
+    float *sm = reinterpret_cast<float *>(sm_raw + A.rec_slots * kAdsRecBytes);
+    AdsShare B;
+    const int64_t b = blockIdx.x, g = gridDim.x;
+    B.s0 = (int)(b * A.spec_count / g);
+    B.s1 = (int)((b + 1) * A.spec_count / g);
+    B.p0 = (int)(b * A.nplain / g);
+    B.p1 = (int)((b + 1) * A.nplain / g);
+    B.ws = (B.s1 - B.s0 + 31) / 32;
+    B.wp = (B.p1 - B.p0 + 31) / 32;
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (2 * B.ws <= nw)
+    {
+        B.pstep = nw - B.ws;
+        B.pj0 = warp < B.ws ? B.wp : warp - B.ws;
+    }
+    else
+    {
+        B.pstep = nw;
+        B.pj0 = (warp + nw - B.ws % nw) % nw;
+    }
+    B.recs = reinterpret_cast<uint4 *>(sm_raw);
+    if (threadIdx.x == 0) s_rmax = 0u;
+    ads_fill(A, B, sm);
+    __syncthreads();
     unsigned int target = 0;
+#pragma unroll 1
     for (int k = 0; k < A.nsteps; k++)
     {
+        const int parity = (A.parity0 + k) & 1;
+        const bool last = k + 1 == A.nsteps, direct = k == 0 && A.direct0;
         StepOpt o{};
-        o.parity = (A.parity0 + k) & 1;
-        o.direct = k == 0 ? A.direct0 : 0;
-        o.red_slot = ((A.slot0 + k) % A.ring) * 4;
-        o.snap_store = 1;
-        StepOpt o1 = o, o2 = o;
-        o1.diff = A.psi_diff;
-        o2.diff = A.step_diff;
-        for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x)
+        o.parity = parity;
+        o.snap_store = last ? 1 : 0; // the outputs show the last step's
+        const float rmax = parity ? ads_pass1<1, FITS>(A, B, sm, direct, last) : ads_pass1<0, FITS>(A, B, sm, direct, last);
+        if (A.psi_diff)
         {
-            float rmax = 0.0f;
-            if (u < A.ntiles) rmax = o.parity ? ads_psi_tile<1>(A.L, A.C, o1, u) : ads_psi_tile<0>(A.L, A.C, o1, u);
-            else
-            {
-                const int i = (u - A.ntiles) * kAdsRecords + (int)threadIdx.x;
-                if (i < A.spec_count)
-                    rmax = o.parity ? ads_psi_record<1>(A.L, A.C, o1, A.spec_begin + i)
-                                    : ads_psi_record<0>(A.L, A.C, o1, A.spec_begin + i);
-            }
-            if (o1.diff) block_max(rmax, A.C.red + o1.red_slot);
+            // non-negative floats order like their bits; a NaN counts as no change
+            const unsigned int v = __reduce_max_sync(0xffffffffu, rmax > 0.0f ? __float_as_uint(rmax) : 0u);
+            if ((threadIdx.x & 31) == 0 && v) atomicMax(&s_rmax, v);
         }
         target += gridDim.x;
-        if (!grid_barrier(A.bar, target, A.C.err)) return;
-        for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x)
-        {
-            double r_diff = 0.0, r_norm = 0.0;
-            if (u < A.ntiles)
-            {
-                if (o.parity) ads_step_tile<1>(A.L, A.C, o2, u, r_diff, r_norm);
-                else ads_step_tile<0>(A.L, A.C, o2, u, r_diff, r_norm);
-            }
-            else
-            {
-                const int i = (u - A.ntiles) * kAdsRecords + (int)threadIdx.x;
-                if (i < A.spec_count)
-                {
-                    if (o.parity) ads_step_record<1>(A.L, A.C, o2, A.spec_begin + i, r_diff, r_norm);
-                    else ads_step_record<0>(A.L, A.C, o2, A.spec_begin + i, r_diff, r_norm);
-                }
-            }
-            if (o2.diff) block_add2(r_diff, r_norm, A.C.red + o2.red_slot);
-        }
+        if (!grid_barrier(A.bar, target, A.C.err, A.psi_diff ? &s_rmax : nullptr,
+                          A.C.red + (size_t)((A.slot0 + k) % A.ring) * 4))
+            return;
+        if (parity) ads_pass2<1, FITS>(A, B, sm, o, direct);
+        else ads_pass2<0, FITS>(A, B, sm, o, direct);
         target += gridDim.x;
-        if (!grid_barrier(A.bar, target, A.C.err)) return;
+        if (!last && !grid_barrier(A.bar, target, A.C.err, nullptr, nullptr)) return;
     }
 }
 

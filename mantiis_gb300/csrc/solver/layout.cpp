@@ -357,6 +357,14 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
         }
     }
 
+    // plain cells in row order, for the adsorption engine that gives each thread
+    // its cells for many steps
+    if (p.adsorption)
+        for (auto &lv : L.levels)
+            for (int y = 0; y < lv.H; y++)
+                for (int x = 0; x < lv.W; x++)
+                    if (lv.omega[(size_t)y * lv.pitch + x] > 0.0f) lv.plain_xy.push_back(x | y << 16);
+
     // 8x4 tiles holding a plain or light cell, row-major (one warp per tile in the
     // 8x4 kernel: sparse levels fill them better than 32x8 tiles), with the mask
     // of their light cells

@@ -79,6 +79,7 @@ struct LevelLayout
     std::vector<int32_t> tile8_list;  // 8x4 tiles holding a plain or light cell: tx | ty << 16 (x in 8s, y in 4s)
     std::vector<uint32_t> tile8_mask; // per such tile, its plain and light cells (bit = 8 * row + column)
     std::vector<uint32_t> tile8_light;// per such tile, its light cells (subset of tile8_mask)
+    std::vector<int32_t> plain_xy;    // plain cells, row-major: x | y << 16 (adsorption only)
     int64_t n_active = 0, n_active_real = 0;
     int substeps = 1;                // per coarse step, 2^(L-l)
     int64_t spec_begin = 0, spec_count = 0; // this level's special records (sorted by site)

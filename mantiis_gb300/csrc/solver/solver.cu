@@ -111,7 +111,7 @@ struct LevelDev
     bool use8 = false;   // plain cells through the 8x4 warp-tile kernel
     DevBuf<float> f, omega, tau2, snap, unorm, psi, rho_prev;
     DevBuf<uint32_t> spec;
-    DevBuf<int32_t> tiles, tiles8;
+    DevBuf<int32_t> tiles, tiles8, plain_xy;
     DevBuf<uint32_t> tile_mask, tile8_mask, tile8_light;
     int64_t steps = 0; // substeps done at this level
 };
@@ -255,7 +255,6 @@ struct mgpu_ctx
     // passes (pairs of steps replayed from a CUDA graph)
     int engine = MGPU_ENGINE_PERSISTENT;
     DevBuf<unsigned int> ads_bar; // grid-barrier arrivals of k_ads_persistent
-    int ads_grid = 0;             // its blocks: all resident at once
     float rho0f = 0.f;
     bool adsorption = false; // Shan-Chen step body (include/mantiisApp.hpp:248-265)
     // coupled run (include/mantiisApp.hpp:376-392): up to 100 adsorption steps
@@ -803,29 +802,48 @@ void run_ads_persistent(mgpu_ctx *ctx, int n, int64_t k, bool diff)
     dev::AdsPersist A{};
     A.L = ctx->view(0);
     A.C = ctx->common();
+    A.plain_xy = ctx->lv[0].plain_xy.p;
+    A.nplain = (int)ll.plain_xy.size();
     A.spec_begin = ll.spec_begin;
     A.spec_count = (int)ll.spec_count;
-    A.ntiles = (int)ll.tile_list.size();
     A.nsteps = n;
     A.parity0 = (int)(ctx->lv[0].steps & 1);
     A.direct0 = ctx->lv[0].steps == 0 ? 1 : 0;
     A.slot0 = (int)(k % kRing);
     A.ring = kRing;
     A.psi_diff = diff ? 1 : 0; // the density change (the coupling phase, with |u| sums, is not run here)
-    A.step_diff = 0;
     A.bar = ctx->ads_bar.p;
-    const int units = A.ntiles + (A.spec_count + dev::kAdsRecords - 1) / dev::kAdsRecords;
-    if (ctx->ads_grid == 0)
-    {
-        int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_ads_persistent, 256, 0));
-        ctx->ads_grid = std::max(1, per_sm) * ctx->sm_count;
-    }
-    const int grid = std::min(units, ctx->ads_grid);
+    // one block per SM with at least four warps of cells each; the warps of a
+    // block share its warps of cells evenly, as much of their data as fits in
+    // shared memory
+    const int warps = (A.nplain + 31) / 32 + (A.spec_count + 31) / 32;
+    const int grid = std::max(1, std::min(ctx->sm_count, warps / 4));
+    const int ws = (A.spec_count / grid + 32) / 32, wp = (A.nplain / grid + 32) / 32, per_block = ws + wp;
+    const bool small = per_block * 32 <= dev::kAdsSmall;
+    const int most = (small ? dev::kAdsSmall : dev::kAdsLarge) / 32;
+    int warps_of_block = std::min(per_block, most);
+    if (2 * ws <= most)
+        for (int rounds = 1; rounds <= wp; rounds++)
+            if (ws + (wp + rounds - 1) / rounds <= most)
+            {
+                warps_of_block = ws + (wp + rounds - 1) / rounds;
+                break;
+            }
+    const int threads = warps_of_block * 32;
+    int smem_max = 0;
+    CK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    size_t room = (size_t)smem_max - 1024; // (the kernel's static shared memory)
+    A.rec_slots = std::min(ws, (int)(room / 4 / dev::kAdsRecBytes));
+    room -= (size_t)A.rec_slots * dev::kAdsRecBytes;
+    A.slots = std::min(per_block, (int)(room / dev::kAdsSlotBytes));
+    const size_t smem = (size_t)A.rec_slots * dev::kAdsRecBytes + (size_t)A.slots * dev::kAdsSlotBytes;
+    const void *kernel = A.slots < per_block ? (const void *)dev::k_ads_persistent<dev::kAdsLarge, false>
+                         : small             ? (const void *)dev::k_ads_persistent<dev::kAdsSmall, true>
+                                             : (const void *)dev::k_ads_persistent<dev::kAdsLarge, true>;
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 1024));
     CK(cudaMemsetAsync(A.bar, 0, sizeof(unsigned int), ctx->stream));
     void *args[] = {&A};
-    CK(cudaLaunchCooperativeKernel((const void *)dev::k_ads_persistent, dim3((unsigned)grid), dim3(256), args, 0,
-                                   ctx->stream));
+    CK(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)grid), dim3((unsigned)threads), args, smem, ctx->stream));
     ctx->launches++;
     ctx->lv[0].steps += n;
     ctx->coarse_done += n;
@@ -1544,6 +1562,7 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
         d.tiles.upload(ll.tile_list, acct, s);
         d.tile_mask.upload(ll.tile_mask, acct, s);
         d.tiles8.upload(ll.tile8_list, acct, s);
+        d.plain_xy.upload(ll.plain_xy, acct, s);
         d.tile8_mask.upload(ll.tile8_mask, acct, s);
         d.tile8_light.upload(ll.tile8_light, acct, s);
         d.use8 = p->plain_path == 2 && !ctx->adsorption;
