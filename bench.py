@@ -539,8 +539,9 @@ def main():
                     help="repeat the timed K-step window until the windows cover this much time")
     ap.add_argument("--steady-images", type=int, default=4,
                     help="images of the steady-state leg (0 = skip it)")
-    ap.add_argument("--engine", type=int, default=0, choices=[0, 1],
-                    help="batch engine: 0 per-image launches on concurrent streams, 1 one persistent launch per step")
+    ap.add_argument("--engine", type=int, default=-1, choices=[-1, 0, 1],
+                    help="batch engine: -1 the library's choice, 0 per-image launches on concurrent streams, "
+                         "1 one persistent launch per step")
     ap.add_argument("--steady-batch", type=int, default=0,
                     help="also run this many config4_steady images to steady state as one batch")
     ap.add_argument("--workload", default="config2", choices=sorted(WORKLOADS))
@@ -600,11 +601,11 @@ def main():
     lu_step = float(sum(s.info["lu_per_step"] for s in solvers))
     state_mb = sum(s.info["device_bytes"] for s in solvers) / 1e6
 
-    # all images step together: one launch per phase over the batch, two
-    # coarse steps per CUDA graph (captured during the warm-up)
+    # all images step together by the library's choice of engine (--engine)
     batch = Batch(solvers)
     batch.set_stream(stream.cuda_stream)
-    batch.set_engine(args.engine, 0)
+    if args.engine >= 0:
+        batch.set_engine(args.engine, 0)
     warm = args.warmup + (args.warmup % 2)
     batch.advance(warm)
     torch.cuda.synchronize()
@@ -757,10 +758,14 @@ def main():
                        "n": [int(im["pore"].shape[0]) for im in imgs] if args.workload == "config4" else 1024,
                        "levels": [int(im["levels"]) for im in imgs] if args.workload == "config4" else imgs[0]["levels"],
                        "lu_per_step_per_gpu": lu_step, "device_state_mb_per_gpu": round(state_mb, 1),
-                       "l2": "inputs larger than L2 (state of the batch > 129 MB)",
-                       "graph": ("one CUDA graph of 2 coarse steps for the whole batch, images on L2-sized concurrent "
-                                 "streams" if args.engine == 0 else
-                                 "one CUDA graph of 2 coarse steps for the whole batch, one persistent launch per step"),
+                       "l2": "inputs larger than L2 (state of the batch > 129 MB)" +
+                             ("; a cooperative launch steps one L2-sized group of images up to 500 times"
+                              if args.engine < 0 else ""),
+                       "graph": {-1: "cooperative launches of up to 500 coarse steps per group of images",
+                                 0: "one CUDA graph of 2 coarse steps for the whole batch, images on L2-sized "
+                                    "concurrent streams",
+                                 1: "one CUDA graph of 2 coarse steps for the whole batch, one persistent launch "
+                                    "per step"}[args.engine],
                        "state_finite_after_timed_steps": finite,
                        **({} if finite else {"state_note": "the reference's multi-block scheme diverges on these "
                                                            "images (its FP64 restatement too); the step's work "

@@ -242,17 +242,22 @@ int mgpu_batch_set_stream(mgpu_batch *b, void *stream);
  * of the batch: blocks claim units of work in order and a stage of an image
  * (a phase of its coarse step, an interface wave) starts when its previous
  * stage is complete, as device-side counters show; `group` images (0 = all)
- * are interleaved at a time.  Both engines give bit-identical states. */
+ * are interleaved at a time.  Until this is called, a batch whose images are
+ * small enough (state of up to twice the L2 each) steps groups of images in
+ * cooperative launches of many coarse steps, as single contexts do
+ * (mgpu_set_engine), others by engine 0.  All give bit-identical states. */
 #define MGPU_ENGINE_STREAMS 0
 #define MGPU_ENGINE_PERSISTENT 1
 int mgpu_batch_set_engine(mgpu_batch *b, int engine, int group);
-/* The adsorption step of one context (single level, not coupled): engine 1
- * (the default) runs the steps of an mgpu_run batch, an mgpu_advance call or an
- * mgpu_advance_graph call in one cooperative launch, all of its blocks resident,
- * each of the two passes of a step closed by a grid barrier whose waits are
- * bounded (about a second, then MGPU_E_DEVICE); engine 0 launches the passes of
- * every step (pairs of steps replayed from a CUDA graph).  Both give
- * bit-identical states; transport contexts are not affected. */
+/* How one context steps: engine 1 (the default) runs the steps of an mgpu_run
+ * batch, an mgpu_advance call or an mgpu_advance_graph call in cooperative
+ * launches of many steps, all of their blocks resident, each pass of an
+ * adsorption step (single level, not coupled) and each phase and interface wave of
+ * a transport step closed by a grid barrier whose waits are bounded (some
+ * seconds, then MGPU_E_DEVICE); engine 0 launches the passes or phases of every
+ * step (pairs of steps replayed from a CUDA graph).  Both give bit-identical
+ * states.  A transport context uses engine 0 all the same where plain_path names a
+ * kernel of it or `concurrent` says that other contexts share the GPU. */
 int mgpu_set_engine(mgpu_ctx *ctx, int engine);
 int mgpu_batch_sync(mgpu_batch *b);
 int64_t mgpu_batch_launch_count(const mgpu_batch *b);

@@ -363,16 +363,16 @@ template <int P> __device__ __forceinline__ float wall_slot(const LevelView &L, 
 // (include/mantiisApp.hpp:239-265, include/coreLB.hpp:834-1009).  `raw` holds
 // the slots the cell reads at parity P; `wall(q)` gives the value its wall
 // link q left in the previous step.
-template <int P, typename WallSlot>
-__device__ __forceinline__ void special_rules(const Common &C, const SpecialRec &rec, const float raw[9], WallSlot wall_of,
-                                              float df[9])
+template <typename WallSlot>
+__device__ __forceinline__ void special_rules(const Common &C, const SpecialRec &rec, int parity, int wall_mode,
+                                              const float raw[9], WallSlot wall_of, float df[9])
 {
     const uint32_t arrive = rec.m0 & 0x1FFu, over = (rec.m0 >> 9) & 0x1FFu, wall = (rec.m0 >> 18) & 0x1FFu;
     const uint32_t quirk = rec.m1 & 0x1FFu, bnd = (rec.m1 >> 9) & 0xFFu, flags = (rec.m1 >> 17) & 0xFu;
     // every load first (wall values, quirk values, constant terms, specular
     // targets), so they are in flight together; then the arithmetic in the
     // reference's order
-    const float *side_prev = C.side + (size_t)(P ^ 1) * C.n_quirk;
+    const float *side_prev = C.side + (size_t)(parity ^ 1) * C.n_quirk;
     float v[9], kq[9];
     int p2s[9];
 #pragma unroll
@@ -402,7 +402,7 @@ __device__ __forceinline__ void special_rules(const Common &C, const SpecialRec 
         {
             if (!((wall >> q) & 1u)) continue;
             const int p1 = d2q9::opp(q);
-            if (C.wall == WALL_SRBB)
+            if (wall_mode == WALL_SRBB)
             {
                 const int p2 = p2s[q];
                 if (!((over >> p1) & 1u)) df[p1] += r * v[q];
@@ -438,7 +438,7 @@ __device__ __forceinline__ void load_special(const LevelView &L, const Common &C
 {
     float raw[9];
     load_raw<P>(L, x, y, raw);
-    special_rules<P>(C, rec, raw, [&](int q) { return wall_slot<P>(L, x, y, q); }, df);
+    special_rules(C, rec, P, C.wall, raw, [&](int q) { return wall_slot<P>(L, x, y, q); }, df);
 }
 } // namespace dev
 } // namespace mantiis

@@ -95,6 +95,66 @@ template <bool NC> __device__ __forceinline__ void load_snap(const LevelView &L,
     sn[2] = ldf<NC>(&L.snap[2 * L.plane + s]);
 }
 
+// Collision of one cell with the populations df: equilibrium of the moments
+// edrho, erho, eux, euy (the cell's own, or those of the coarse step's start),
+// regularized MRT / MRT / BGK, the wall values of special cells
+// (include/coreLB.hpp:420-430, 646-792, 834-977).  fs: the populations to stream.
+__device__ __forceinline__ void collide_cell(const LevelView &L, const Common &C, int collision, int wall_mode, int parity,
+                                             int64_t s, const float df[9], float edrho, float erho, float eux, float euy,
+                                             float omega, bool special, const SpecialRec &rec, float fs[9])
+{
+    float feq[9];
+    equilibrium(edrho, erho, eux, euy, feq);
+    if (collision == COLL_RMRT) collide_rmrt(df, feq, edrho, erho, eux, euy, omega, fs);
+    else if (collision == COLL_MRT) collide_mrt(df, feq, mrt_rates(1.0f / omega, L.tau2 ? L.tau2[s] : 1.0f), fs);
+    else
+    {
+        const float inv_tau = 1.0f; // 1 / tau_SRT, tau_SRT = 1 (include/globalParameters.hpp:140)
+#pragma unroll
+        for (int q = 0; q < 9; q++) fs[q] = df[q] - inv_tau * (df[q] - feq[q]);
+    }
+    if (special)
+    {
+        const uint32_t wall = (rec.m0 >> 18) & 0x1FFu, quirk = rec.m1 & 0x1FFu;
+        if (wall && wall_mode == WALL_MDBB)
+        {
+            // include/coreLB.hpp:936-967: reflected value
+            //   r f*_q + (1 - r) (sum_{c.n<0} f / sum_{c.n>0} f_eq) f_eq,opp(q)
+            // in deviation form; both sums share the weight total A.
+            const uint32_t bnd = (rec.m1 >> 9) & 0xFFu;
+            const uint32_t pos = bnd == 0xFFu ? 0u : c_npos[bnd], neg = bnd == 0xFFu ? 0u : c_nneg[bnd];
+            float a = 0.f, ap = 0.f, A = 0.f;
+#pragma unroll
+            for (int q = 0; q < 9; q++)
+            {
+                if ((neg >> q) & 1u) a += df[q];
+                if ((pos >> q) & 1u)
+                {
+                    ap += feq[q];
+                    A += wq(q) * C.rho0;
+                }
+            }
+            const float g = (A + ap) != 0.f ? (a - ap) / (A + ap) : 0.f;
+            const float r = rec.r;
+#pragma unroll
+            for (int q = 0; q < 9; q++)
+                if ((wall >> q) & 1u)
+                {
+                    const int po = d2q9::opp(q);
+                    fs[q] = r * fs[q] + (1.0f - r) * (feq[po] + (wq(po) * C.rho0 + feq[po]) * g);
+                }
+        }
+        if (quirk)
+        {
+            float *side_now = C.side + (size_t)parity * C.n_quirk;
+            int qi = 0;
+#pragma unroll
+            for (int q = 0; q < 9; q++)
+                if ((quirk >> q) & 1u) side_now[rec.quirk_base + qi++] = fs[q];
+        }
+    }
+}
+
 // Collision and streaming of one cell whose populations df are loaded:
 // macroscopic moments (and the residual / snapshot side outputs), equilibrium,
 // regularized MRT / MRT / BGK collision, the wall values of special cells and
@@ -133,56 +193,8 @@ __device__ __forceinline__ void step_cell(const LevelView &L, const Common &C, c
         eux = snap_prev ? snap_prev[1] : L.snap[L.plane + s];
         euy = snap_prev ? snap_prev[2] : L.snap[2 * L.plane + s];
     }
-    float feq[9], fs[9];
-    equilibrium(edrho, erho, eux, euy, feq);
-    if (C.collision == COLL_RMRT) collide_rmrt(df, feq, edrho, erho, eux, euy, omega, fs);
-    else if (C.collision == COLL_MRT) collide_mrt(df, feq, mrt_rates(1.0f / omega, L.tau2 ? L.tau2[s] : 1.0f), fs);
-    else
-    {
-        const float inv_tau = 1.0f; // 1 / tau_SRT, tau_SRT = 1 (include/globalParameters.hpp:140)
-#pragma unroll
-        for (int q = 0; q < 9; q++) fs[q] = df[q] - inv_tau * (df[q] - feq[q]);
-    }
-    if (special)
-    {
-        const uint32_t wall = (rec.m0 >> 18) & 0x1FFu, quirk = rec.m1 & 0x1FFu;
-        if (wall && C.wall == WALL_MDBB)
-        {
-            // include/coreLB.hpp:936-967: reflected value
-            //   r f*_q + (1 - r) (sum_{c.n<0} f / sum_{c.n>0} f_eq) f_eq,opp(q)
-            // in deviation form; both sums share the weight total A.
-            const uint32_t bnd = (rec.m1 >> 9) & 0xFFu;
-            const uint32_t pos = bnd == 0xFFu ? 0u : c_npos[bnd], neg = bnd == 0xFFu ? 0u : c_nneg[bnd];
-            float a = 0.f, ap = 0.f, A = 0.f;
-#pragma unroll
-            for (int q = 0; q < 9; q++)
-            {
-                if ((neg >> q) & 1u) a += df[q];
-                if ((pos >> q) & 1u)
-                {
-                    ap += feq[q];
-                    A += wq(q) * C.rho0;
-                }
-            }
-            const float g = (A + ap) != 0.f ? (a - ap) / (A + ap) : 0.f;
-            const float r = rec.r;
-#pragma unroll
-            for (int q = 0; q < 9; q++)
-                if ((wall >> q) & 1u)
-                {
-                    const int po = d2q9::opp(q);
-                    fs[q] = r * fs[q] + (1.0f - r) * (feq[po] + (wq(po) * C.rho0 + feq[po]) * g);
-                }
-        }
-        if (quirk)
-        {
-            float *side_now = C.side + (size_t)P * C.n_quirk;
-            int qi = 0;
-#pragma unroll
-            for (int q = 0; q < 9; q++)
-                if ((quirk >> q) & 1u) side_now[rec.quirk_base + qi++] = fs[q];
-        }
-    }
+    float fs[9];
+    collide_cell(L, C, C.collision, C.wall, P, s, df, edrho, erho, eux, euy, omega, special, rec, fs);
     store_post<P>(L, x, y, fs, interior);
 }
 
@@ -217,6 +229,22 @@ __device__ __forceinline__ void plain_tile(const LevelView &L, const Common &C, 
         SpecialRec none;
         step_cell<P>(L, C, o, diff, store_u, x, y, s, df, om, false, none, r_diff, r_norm, interior, &uprev,
                      o.snap_use ? sn : nullptr);
+    }
+}
+
+// Populations of a light cell (special only through missing arrivals and buffer
+// status) from the slots it reads
+__device__ __forceinline__ void light_rules(const Common &C, const SpecialRec &rec, float df[9])
+{
+    const uint32_t arrive = rec.m0 & 0x1FFu;
+    const bool has_k = ((rec.m1 >> 17) & SF_HAS_K) != 0;
+    const float *k = C.ktab + (size_t)(has_k ? rec.k_row : 0) * 9;
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+    {
+        float v = ((arrive >> q) & 1u) ? df[q] : 0.0f;
+        if (has_k) v += __ldg(&k[q]);
+        df[q] = v;
     }
 }
 
@@ -257,7 +285,7 @@ __device__ __forceinline__ void plain_tile8(const LevelView &L, const Common &C,
     else
     {
         const SpecialRec rec = C.specials[__ldg(&L.spec[s])];
-        const uint32_t arrive = rec.m0 & 0x1FFu, flags = (rec.m1 >> 17) & 0xFu;
+        const uint32_t flags = (rec.m1 >> 17) & 0xFu;
         om = rec.omega;
         if ((flags & SF_BUFFER) && (o.first_sub || o.direct))
         {
@@ -268,18 +296,7 @@ __device__ __forceinline__ void plain_tile8(const LevelView &L, const Common &C,
         {
             // a direct state has parity 0: own slots, as load_raw<0>
             load_raw_ro<P, NC>(L, x, y, df, interior);
-            if (!o.direct)
-            {
-                const bool has_k = (flags & SF_HAS_K) != 0;
-                const float *k = C.ktab + (size_t)(has_k ? rec.k_row : 0) * 9;
-#pragma unroll
-                for (int q = 0; q < 9; q++)
-                {
-                    float v = ((arrive >> q) & 1u) ? df[q] : 0.0f;
-                    if (has_k) v += __ldg(&k[q]);
-                    df[q] = v;
-                }
-            }
+            if (!o.direct) light_rules(C, rec, df);
         }
     }
     SpecialRec none;
@@ -904,13 +921,20 @@ __device__ __forceinline__ void store_for_load(const LevelView &L, int x, int y,
 
 // populations of an interface source cell: its interpolation buffer, or the
 // cell's own slots after streaming and its rules
+// (`plain`: the row has no special source, which holds for all but a few rows;
+// its cells' rates need not be looked up before their populations)
 template <int P>
-__device__ __forceinline__ void load_source(const LevelView &L, const Common &C, int site, int buf, float z[9])
+__device__ __forceinline__ void load_source(const LevelView &L, const Common &C, int site, int buf, bool plain, float z[9])
 {
     if (buf >= 0)
     {
 #pragma unroll
         for (int q = 0; q < 9; q++) z[q] = C.ibuf[(size_t)q * C.n_buf + buf];
+    }
+    else if (plain)
+    {
+        const int x = site % L.pitch, y = site / L.pitch;
+        load_raw_ro<P, false>(L, x, y, z, x > 0 && x + 1 < L.W && y > 0 && y + 1 < L.H);
     }
     else
     {
@@ -930,7 +954,7 @@ __device__ __forceinline__ void coarse_row(const LevelView &Lf, const LevelView 
     const int lane = threadIdx.x & 31, base = lane & ~3;
     const bool has = valid && row.child[k] >= 0;
     float df[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (has) load_source<PF>(Lf, C, row.child[k], row.child_buf[k], df);
+    if (has) load_source<PF>(Lf, C, row.child[k], row.child_buf[k], !row.special, df);
     float mean[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
     for (int kk = 0; kk < 4; kk++)
@@ -969,8 +993,8 @@ __device__ __forceinline__ void fine_child(const LevelView &Lf, const LevelView 
     float za[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, zb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (valid)
     {
-        load_source<PC>(Lc, C, row.node_site[c], row.node_buf[c], za);
-        if (c < 2) load_source<PC>(Lc, C, row.node_site[c + 4], row.node_buf[c + 4], zb);
+        load_source<PC>(Lc, C, row.node_site[c], row.node_buf[c], !row.special, za);
+        if (c < 2) load_source<PC>(Lc, C, row.node_site[c + 4], row.node_buf[c + 4], !row.special, zb);
     }
     float acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
@@ -1257,7 +1281,7 @@ struct AdsPersist
 {
     LevelView L;
     Common C;
-    const int32_t *plain_xy; // plain cells, row-major: x | y << 16
+    const int32_t *plain_xy; // plain cells: x | y << 16
     int64_t spec_begin;
     int nplain, spec_count;
     int slots;              // cells' warps whose data fits a block's shared memory
@@ -1284,16 +1308,48 @@ constexpr size_t kAdsRecBytes = (size_t)32 * sizeof(SpecialRec); // records of o
 // 512 threads (128 registers, nothing spilled), the others that of up to 640 (96)
 constexpr int kAdsSmall = 512, kAdsLarge = 640;
 
+// Sums of a and b over each warp, to sums[warp]; after a block barrier one warp
+// adds the warps' sums to dst[0] and dst[1].
+__device__ __forceinline__ void block_sums(double a, double b, double2 *sums)
+{
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = make_double2(a, b);
+}
+__device__ __forceinline__ void add_block_sums(const double2 *sums, double *dst)
+{
+    const int lane = threadIdx.x & 31;
+    double2 v = lane < (int)(blockDim.x >> 5) ? sums[lane] : make_double2(0.0, 0.0);
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+    }
+    if (lane == 0)
+    {
+        if (v.x != 0.0) atomicAdd(dst, v.x);
+        if (v.y != 0.0) atomicAdd(dst + 1, v.y);
+    }
+}
+
 // Grid barrier `target` = (barriers passed) x gridDim.x: every block adds one
 // arrival with release semantics after its block barrier, then waits (bounded)
 // for all of them; a wait that runs out sets the error word and the block stops.
 // rmax: if not null, the block's maximum of the residual terms (non-negative
-// floats by their bit patterns), which goes to dst and is cleared.
+// floats by their bit patterns), which goes to dst and is cleared; clear: a
+// counter in shared memory set to zero on the way; sums: if not null, the warps'
+// pairs of sums in shared memory (block_sums), which warp 1 adds to sums_to while
+// the block waits.
 __device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int target, unsigned int *err,
-                                             unsigned int *rmax, double *dst)
+                                             unsigned int *rmax, double *dst, unsigned int *clear = nullptr,
+                                             const double2 *sums = nullptr, double *sums_to = nullptr)
 {
     __shared__ int s_ok;
     __syncthreads();
+    if (sums && threadIdx.x >= 32 && threadIdx.x < 64) add_block_sums(sums, sums_to);
     if (threadIdx.x == 0)
     {
         if (rmax && *rmax)
@@ -1302,6 +1358,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int tar
                       (unsigned long long)__double_as_longlong((double)__uint_as_float(*rmax)));
             *rmax = 0u;
         }
+        if (clear) *clear = 0u;
         add_release(bar, 1u);
         bool ok = false;
         for (uint32_t i = 0; i < kDepPolls && !ok; i++)
@@ -1605,6 +1662,732 @@ __global__ void __launch_bounds__(THREADS, 1) k_ads_persistent(const __grid_cons
         else ads_pass2<0, FITS>(A, B, sm, o, direct);
         target += gridDim.x;
         if (!last && !grid_barrier(A.bar, target, A.C.err, nullptr, nullptr)) return;
+    }
+}
+
+// ---- transport steps of a group of images as one cooperative launch over many
+// coarse steps.  The stages of a coarse step are those of the phase engine (a
+// phase steps every level whose next substep falls on it; the interface waves
+// follow), each closed by a grid barrier, over all images of the group; the
+// per-cell arithmetic is the same code, so the states are bit-identical.
+//
+// A stage of the phase engine costs a launch (2 us and more with its fork to the
+// special cells' stream), blocks that fetch a descriptor, a tile and its masks
+// before their first population, and 23 % idle lanes.  Here one block per SM
+// owns the same warps of cells in every step (compacted lists of the cells of
+// each kind and level, an equal share of each): what identifies a cell (position
+// and relaxation rate, or its record), the |u| of the residual and the
+// coarse-step-start moments that only the cell itself reads wait in shared
+// memory.  A cell's populations are then the only round trip to memory.
+//
+// Measured on a GB300, us per coarse step without / with residuals: single block
+// 64^2 4.4 / 5.5, 128^2 4.8 / 5.9, 512^2 6.3 / 7.6, 1024^2 12.3 / 16.2, two levels
+// 256^2 18.6 / 20.0, 1024^2 34 / 37; the launches per phase 6.1 / 10.7, 6.2 / 10.4,
+// 9.3 / 17.4, 16.4 / 34.7, 22.9 / 27.5, 42.8 / 55.9.  A grid barrier takes 0.85 us,
+// a warp of special cells about 3.5: what small images wait for.  At 1024^2 the
+// stages move 1.7 (single block) to 4 times (two levels: thin bands of fine cells)
+// the cells' bytes, whole sectors, between L2 and the SMs.
+constexpr int kMaxCoopDescs = 40, kMaxCoopPairs = 30;
+
+enum CoopKind
+{
+    CK_HEAVY = 0, // special records with walls, periodic overrides, ...
+    CK_LIGHT = 1, // special records with missing arrivals or buffer status only
+    CK_EDGE = 2,  // plain buffer cells: the interface waves read their coarse-step-start moments
+    CK_PLAIN = 3, // other plain cells
+    CK_KINDS = 4,
+};
+
+struct CoopDesc // one level of one image
+{
+    LevelView L;
+    Common C;
+    const int32_t *xy[CK_KINDS]; // plain cells of the two kinds: x | y << 16
+    int64_t spec_begin;      // the level's records: the heavy ones, then the light ones
+    const int32_t *cut[CK_KINDS]; // block b steps cells [cut[b], cut[b + 1]) of each kind
+    int nheavy;              // records before the light ones
+    int lines[CK_KINDS];     // shared-memory lines per warp of cells
+    int shift;               // steps in the phases that are multiples of 1 << shift
+    int substeps, parity0, direct0, mb;
+};
+
+struct CoopPair // one level pair of one image
+{
+    const CoarseRowDev *coarse;
+    const FineRowDev *fine;
+    int ncoarse, nfine;
+    int df, dc; // descriptors of its fine / coarse level
+    int l1;     // 1 for levels (1, 2), ...
+    int rot;
+};
+
+struct CoopLaunch
+{
+    int nd, np, nphase, nwave;
+    int nsteps;
+    // residual (one image): |u| stored by steps whose number is a multiple of
+    // `every`, compared by the step after, into slot (number of the storing step) mod
+    // ring; skip_first: not by the launch's first step, whose number mod `every` is
+    // since0 and whose predecessor's slot is slot0
+    int every, skip_first, ring, since0, slot0;
+    unsigned int *bar, *err; // grid-barrier arrivals (zero at launch), error word
+    CoopDesc d[kMaxCoopDescs];
+    CoopPair p[kMaxCoopPairs];
+};
+
+// W warps of interface rows dealt to G blocks: block b takes [cut(b), cut(b + 1));
+// the rotation spreads the lists' remainders over the blocks.
+__host__ __device__ inline int coop_cut(int W, int rot, int b, int G) { return (int)(((int64_t)W * b + rot) / G); }
+
+// Shared memory in lines of 32 words (one per lane).  A plain warp of cells: the
+// site (coop_site), 1/tau_s, |u|, and for CK_PLAIN on levels of several substeps
+// the coarse-step-start moments; a special one: its records (two 16-byte halves),
+// |u|.
+constexpr int kCoopPlainLines = 3, kCoopSnapLines = 3, kCoopRecLines = 9;
+constexpr uint32_t kCoopNone = 0xFFFFFFFFu; // a lane past the list
+
+// site of cell (x, y) in the lower 28 bits, above it which of the level's borders
+// the cell lies on: its neighbours there wrap around the torus
+constexpr uint32_t kCoopSite = (1u << 28) - 1u, kCoopLeft = 1u << 28, kCoopRight = 1u << 29, kCoopLow = 1u << 30,
+                   kCoopHigh = 1u << 31;
+__device__ __forceinline__ uint32_t coop_site(const LevelView &L, int x, int y)
+{
+    return (uint32_t)site_of(L, x, y) | (x == 0 ? kCoopLeft : 0u) | (x + 1 == L.W ? kCoopRight : 0u) |
+           (y == 0 ? kCoopLow : 0u) | (y + 1 == L.H ? kCoopHigh : 0u);
+}
+
+struct CoopRange // a block's cells of one kind and level, or rows (lo in warps)
+{
+    int lo, cells; // first cell, cells
+    int n, line;   // warps of cells or rows, first line
+};
+
+// Slots of a cell.  A step reads and writes the same nine: on plane p its own
+// site's (even step) or that of the site at +c_p (odd step); they hold the
+// populations p / opp(p) before and opp(p) / p after the step.  The plane and row
+// strides are read anew per cell (volatile): nine plane offsets kept in registers
+// over the loops would cost the kernel a third of its warps.
+struct CoopSlots
+{
+    float *f;
+    uint32_t at[9];
+    int par;
+    __device__ __forceinline__ CoopSlots(const LevelView &L, const volatile uint2 *stride, uint32_t site, int parity)
+        : f(L.f), par(parity)
+    {
+        const uint32_t plane = stride->x, s = site & kCoopSite;
+        uint32_t up = stride->y, down = 0u - up, right = 1u, left = 0u - 1u;
+        if (site & ~kCoopSite)
+        {
+            if (site & kCoopHigh) up -= (uint32_t)L.H * up;
+            if (site & kCoopLow) down += (uint32_t)L.H * stride->y;
+            if (site & kCoopRight) right -= (uint32_t)L.W;
+            if (site & kCoopLeft) left += (uint32_t)L.W;
+        }
+        if (!par) up = down = right = left = 0u;
+#pragma unroll
+        for (int p = 0; p < 9; p++)
+            at[p] = s + (d2q9::cy(p) > 0 ? up : d2q9::cy(p) < 0 ? down : 0u) +
+                    (d2q9::cx(p) > 0 ? right : d2q9::cx(p) < 0 ? left : 0u) + p * plane;
+    }
+    __device__ __forceinline__ void read(float v[9]) const
+    {
+        float w[9];
+#pragma unroll
+        for (int p = 0; p < 9; p++) w[p] = f[at[p]];
+#pragma unroll
+        for (int q = 0; q < 9; q++) v[q] = par ? w[d2q9::opp(q)] : w[q];
+    }
+    __device__ __forceinline__ void write(const float v[9]) const
+    {
+#pragma unroll
+        for (int p = 0; p < 9; p++) f[at[p]] = par ? v[p] : v[d2q9::opp(p)];
+    }
+    // values into the slots that a step of this parity reads
+    __device__ __forceinline__ void fill(const float v[9]) const
+    {
+#pragma unroll
+        for (int p = 0; p < 9; p++) f[at[p]] = par ? v[d2q9::opp(p)] : v[p];
+    }
+};
+
+struct CoopStep // block-uniform state of one level in one phase
+{
+    StepOpt o;
+    int diff, store_u;
+    int collision, wall;
+};
+
+__device__ __forceinline__ SpecialRec coop_record(const float *line, int lane)
+{
+    union
+    {
+        SpecialRec rec;
+        uint4 v[2];
+    } t;
+    static_assert(sizeof(SpecialRec) == 2 * sizeof(uint4), "record size");
+    t.v[0] = reinterpret_cast<const uint4 *>(line)[lane];
+    t.v[1] = reinterpret_cast<const uint4 *>(line)[32 + lane];
+    return t.rec;
+}
+
+// Moments, residual and collision of a cell with the populations df.  snap: where
+// its coarse-step-start moments are kept, three values `stride` apart; sn: these,
+// loaded ahead (snap_use).
+template <bool SPECIAL, bool RES>
+__device__ __forceinline__ void coop_collide(const CoopDesc &D, const CoopStep &st, int64_t s, const float df[9], float *snap,
+                                             int64_t stride, const float sn[3], float omega, const SpecialRec &rec,
+                                             float *unorm, double2 *acc, float fs[9])
+{
+    float drho, rho, ux, uy;
+    macro(df, D.C.rho0, D.L.fshift, 0.0f, drho, rho, ux, uy);
+    if (RES && (st.diff | st.store_u))
+    {
+        const float un = sqrtf(ux * ux + uy * uy);
+        if (st.diff)
+        {
+            double2 v = *acc;
+            v.x += (double)fabsf(un - *unorm);
+            v.y += (double)un;
+            *acc = v;
+        }
+        if (st.store_u) *unorm = un;
+    }
+    if (st.o.snap_store && snap)
+    {
+        snap[0] = drho;
+        snap[stride] = ux;
+        snap[2 * stride] = uy;
+    }
+    float edrho = drho, erho = rho, eux = ux, euy = uy;
+    if (st.o.snap_use)
+    {
+        edrho = sn[0];
+        erho = D.C.rho0 + edrho;
+        eux = sn[1];
+        euy = sn[2];
+    }
+    collide_cell(D.L, D.C, st.collision, st.wall, st.o.parity, s, df, edrho, erho, eux, euy, omega, SPECIAL, rec, fs);
+}
+
+// One special cell from its record.
+template <bool HEAVY, bool RES>
+__device__ __forceinline__ void coop_special(const CoopDesc &D, const CoopStep &st, const volatile uint2 *stride,
+                                             const SpecialRec &rec, float *unorm, double2 *acc)
+{
+    const LevelView &L = D.L;
+    const int x = rec.xy & 0xFFFF, y = rec.xy >> 16;
+    const int64_t s = site_of(L, x, y);
+    const int par = st.o.parity;
+    const uint32_t site = coop_site(L, x, y);
+    float sn[3] = {0.f, 0.f, 0.f}, df[9], fs[9];
+    if (st.o.snap_use) load_snap<false>(L, s, sn);
+    if (((rec.m1 >> 17) & SF_BUFFER) && (st.o.first_sub || st.o.direct))
+    {
+#pragma unroll
+        for (int q = 0; q < 9; q++) df[q] = D.C.ibuf[(size_t)q * D.C.n_buf + rec.buf];
+    }
+    else
+    {
+        // (a direct state has parity 0: own slots)
+        float raw[9];
+        CoopSlots(L, stride, site, par).read(raw);
+        if (st.o.direct || !HEAVY)
+        {
+#pragma unroll
+            for (int q = 0; q < 9; q++) df[q] = raw[q];
+            if (!st.o.direct) light_rules(D.C, rec, df);
+        }
+        else
+        {
+            // a wall link's value lies where the previous step stored it
+            const CoopSlots before(L, stride, site, par ^ 1);
+            special_rules(D.C, rec, par, st.wall, raw,
+                          [&](int q) { return L.f[par ? before.at[d2q9::opp(q)] : before.at[q]]; }, df);
+        }
+    }
+    coop_collide<HEAVY, RES>(D, st, s, df, L.snap ? L.snap + s : nullptr, L.plane, sn, rec.omega, rec, unorm, acc, fs);
+    CoopSlots(L, stride, site, par).write(fs);
+}
+
+// The index, hidden from the compiler: descriptor fields are then read where they
+// are used (from the parameter bank) and not held in registers over the loops.
+__device__ __forceinline__ int coop_opaque(int d)
+{
+    asm volatile("" : "+r"(d));
+    return d;
+}
+
+// The warps of a block claim its warps of cells (or rows) of a stage in order from
+// a counter in shared memory, the long ones first: special cells take two to
+// three times as long as plain ones, and a stage ends with its last warp.
+struct CoopClaim
+{
+    unsigned int *next;
+    int base, mine; // items before the current list, this warp's claim
+    __device__ __forceinline__ explicit CoopClaim(unsigned int *counter) : next(counter), base(0) { claim(); }
+    __device__ __forceinline__ void claim()
+    {
+        unsigned int v = 0;
+        if ((threadIdx.x & 31) == 0) v = atomicAdd(next, 1u);
+        mine = (int)__shfl_sync(0xffffffffu, v, 0);
+    }
+};
+
+// One phase of one level over this block's cells.
+template <bool RES>
+__device__ __forceinline__ void coop_level(const CoopLaunch &A, int d, const CoopStep &st, const CoopRange *rng,
+                                           const volatile uint2 *stride, float *sm, CoopClaim &claim, double2 *acc)
+{
+    const int lane = threadIdx.x & 31;
+    {
+        const CoopRange r = rng[CK_HEAVY];
+#pragma unroll 1
+        for (int i; (i = claim.mine - claim.base) < r.n; claim.claim())
+        {
+            const CoopDesc &D = A.d[coop_opaque(d)];
+            const LevelView &L = D.L;
+            if (i * 32 + lane >= r.cells) continue;
+            float *m = sm + (size_t)(r.line + i * kCoopRecLines) * 32;
+            coop_special<true, RES>(D, st, stride, coop_record(m, lane), m + 8 * 32 + lane, acc);
+        }
+        claim.base += r.n;
+    }
+    {
+        const CoopRange r = rng[CK_LIGHT];
+#pragma unroll 1
+        for (int i; (i = claim.mine - claim.base) < r.n; claim.claim())
+        {
+            const CoopDesc &D = A.d[coop_opaque(d)];
+            const LevelView &L = D.L;
+            if (i * 32 + lane >= r.cells) continue;
+            float *m = sm + (size_t)(r.line + i * kCoopRecLines) * 32;
+            coop_special<false, RES>(D, st, stride, coop_record(m, lane), m + 8 * 32 + lane, acc);
+        }
+        claim.base += r.n;
+    }
+    const SpecialRec none{};
+#pragma unroll 1
+    for (int kind = CK_EDGE; kind <= CK_PLAIN; kind++)
+    {
+        // CK_PLAIN keeps its coarse-step-start moments in shared memory (where a
+        // later substep uses them), CK_EDGE in the planes the waves read
+        const CoopRange r = rng[kind];
+        const int lines = A.d[d].lines[kind];
+        const bool own = kind == CK_PLAIN;
+#pragma unroll 1
+        for (int i; (i = claim.mine - claim.base) < r.n; claim.claim())
+        {
+            const CoopDesc &D = A.d[coop_opaque(d)];
+            const LevelView &L = D.L;
+            float *m = sm + (size_t)(r.line + i * lines) * 32 + lane;
+            const uint32_t site = __float_as_uint(m[0]), s = site & kCoopSite;
+            if (site == kCoopNone) continue;
+            float df[9], fs[9], sn[3] = {0.f, 0.f, 0.f};
+            CoopSlots(L, stride, site, st.o.parity).read(df);
+            float *snap = !own ? L.snap + s : lines > kCoopPlainLines ? m + kCoopPlainLines * 32 : nullptr;
+            const int64_t step = own ? 32 : L.plane;
+            if (st.o.snap_use)
+            {
+                sn[0] = snap[0];
+                sn[1] = snap[step];
+                sn[2] = snap[2 * step];
+            }
+            coop_collide<false, RES>(D, st, s, df, snap, step, sn, m[32], none, m + 64, acc, fs);
+            CoopSlots(L, stride, site, st.o.parity).write(fs);
+        }
+        claim.base += r.n;
+    }
+}
+
+// ---- interface waves of the cooperative steps.  The rows' tables wait in shared
+// memory lane by lane (8 rows of 4 lanes to a warp), so the populations and
+// the coarse-step-start moments of a row are one round trip to memory; the
+// arithmetic is that of coarse_row / fine_child, which step the few rows that
+// touch a special source or the level's border.
+constexpr int kCoopCoarseLines = 3, kCoopFineLines = 12;
+constexpr uint32_t kCoopAbsent = 0xFFFFFFFFu, kCoopBuf = 0x80000000u;
+
+// a source or target of a row off the border is known by its site
+__device__ __forceinline__ bool coop_inner_site(const LevelView &L, int site)
+{
+    const int x = site % L.pitch, y = site / L.pitch;
+    return x > 0 && x + 1 < L.W && y > 0 && y + 1 < L.H;
+}
+__device__ __forceinline__ uint32_t coop_source(const LevelView &L, int site, int buf, bool &slow)
+{
+    if (site < 0) return kCoopAbsent;
+    if (buf >= 0) return kCoopBuf | (uint32_t)buf;
+    slow |= !coop_inner_site(L, site);
+    return (uint32_t)site;
+}
+__device__ __forceinline__ void coop_read_source(const LevelView &L, const volatile uint2 *stride, int par, const Common &C,
+                                                 uint32_t src, float z[9])
+{
+    if (src & kCoopBuf)
+    {
+#pragma unroll
+        for (int q = 0; q < 9; q++) z[q] = C.ibuf[(size_t)q * C.n_buf + (src & ~kCoopBuf)];
+    }
+    else CoopSlots(L, stride, src, par).read(z);
+}
+
+// fills the lines of one warp of rows (r: this lane's row, k: its place in the row)
+__device__ __forceinline__ void coop_fill_coarse(const CoopPair &Q, const LevelView &Lf, const LevelView &Lc, int r, int k,
+                                                 float *m)
+{
+    const int lane = threadIdx.x & 31;
+    bool slow = false;
+    uint32_t src = kCoopAbsent, word = 0;
+    if (r < Q.ncoarse)
+    {
+        const CoarseRowDev &row = Q.coarse[r];
+        src = coop_source(Lf, row.child[k], row.child_buf[k], slow);
+        slow |= row.special || (row.plain_target && !coop_inner_site(Lc, row.site));
+        word = k == 0   ? (uint32_t)row.site
+               : k == 1 ? (uint32_t)row.buf | (row.plain_target ? kCoopBuf : 0u)
+               : k == 2 ? __float_as_uint(row.ratio)
+                        : __float_as_uint(row.inv_nchild);
+    }
+    m[lane] = __uint_as_float(src);
+    m[32 + lane] = __uint_as_float(word);
+    m[64 + lane] = __int_as_float(slow);
+}
+__device__ __forceinline__ void coop_fill_fine(const CoopPair &Q, const LevelView &Lf, const LevelView &Lc, int r, int c, float *m)
+{
+    const int lane = threadIdx.x & 31;
+    bool slow = false;
+    uint32_t a = kCoopAbsent, b = kCoopAbsent, at = 0, buf = 0;
+    float w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, ratio = 0.f;
+    if (r < Q.nfine)
+    {
+        const FineRowDev &row = Q.fine[r];
+        a = coop_source(Lc, row.node_site[c], row.node_buf[c], slow);
+        if (c < 2) b = coop_source(Lc, row.node_site[c + 4], row.node_buf[c + 4], slow);
+#pragma unroll
+        for (int j = 0; j < 6; j++) w[j] = row.weight[c][j];
+        ratio = row.ratio[c];
+        at = (uint32_t)row.child_site[c];
+        const bool plain = (row.plain_mask >> c) & 1;
+        buf = (uint32_t)row.child_buf[c] | (plain ? kCoopBuf : 0u);
+        slow |= row.special || (plain && !coop_inner_site(Lf, row.child_site[c]));
+    }
+    m[lane] = __uint_as_float(a);
+    m[32 + lane] = __uint_as_float(b);
+#pragma unroll
+    for (int j = 0; j < 6; j++) m[(2 + j) * 32 + lane] = w[j];
+    m[8 * 32 + lane] = ratio;
+    m[9 * 32 + lane] = __uint_as_float(at);
+    m[10 * 32 + lane] = __uint_as_float(buf);
+    m[11 * 32 + lane] = __int_as_float(slow);
+}
+
+// One level as the waves see it: its view, strides and the parity of its next step
+struct CoopSide
+{
+    const LevelView &L;
+    const volatile uint2 *stride;
+    int par;
+};
+
+// coarse_row for 8 rows of a warp
+__device__ __forceinline__ void coop_coarse(const CoopSide &F, const CoopSide &Cd, const Common &C, const float *m, bool valid)
+{
+    const int lane = threadIdx.x & 31, base = lane & ~3;
+    const uint32_t src = __float_as_uint(m[lane]);
+    const uint4 t = reinterpret_cast<const uint4 *>(m + 32)[lane >> 2];
+    const bool has = src != kCoopAbsent, out = valid && (lane & 3) == 0;
+    float df[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (has) coop_read_source(F.L, F.stride, F.par, C, src, df);
+    float drho = 0.f, ux = 0.f, uy = 0.f;
+    if (out)
+    {
+        const float *sn = Cd.L.snap + t.x;
+        drho = sn[0];
+        ux = sn[Cd.L.plane];
+        uy = sn[2 * Cd.L.plane];
+    }
+    float mean[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int kk = 0; kk < 4; kk++)
+    {
+        const bool present = __shfl_sync(0xffffffffu, has ? 1 : 0, base + kk) != 0;
+#pragma unroll
+        for (int q = 0; q < 9; q++)
+        {
+            const float v = __shfl_sync(0xffffffffu, df[q], base + kk);
+            if (present) mean[q] += v;
+        }
+    }
+    if (!out) return;
+    float feq[9];
+    equilibrium(drho, C.rho0 + drho, ux, uy, feq);
+    const uint32_t buf = t.y & ~kCoopBuf;
+    const float ratio = __uint_as_float(t.z), inv_nchild = __uint_as_float(t.w);
+    float v[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+    {
+        v[q] = feq[q] + ratio * (mean[q] * inv_nchild - feq[q]);
+        C.ibuf[(size_t)q * C.n_buf + buf] = v[q];
+    }
+    if (t.y & kCoopBuf) CoopSlots(Cd.L, Cd.stride, t.x, Cd.par).fill(v);
+}
+
+// fine_child for 8 rows of a warp
+__device__ __forceinline__ void coop_fine(const CoopSide &F, const CoopSide &Cd, const Common &C, const float *m, bool valid)
+{
+    const int lane = threadIdx.x & 31, base = lane & ~3;
+    const uint32_t a = __float_as_uint(m[lane]), b = __float_as_uint(m[32 + lane]);
+    const uint32_t at = __float_as_uint(m[9 * 32 + lane]), buf = __float_as_uint(m[10 * 32 + lane]);
+    float za[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, zb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (a != kCoopAbsent) coop_read_source(Cd.L, Cd.stride, Cd.par, C, a, za);
+    if (b != kCoopAbsent) coop_read_source(Cd.L, Cd.stride, Cd.par, C, b, zb);
+    float drho = 0.f, ux = 0.f, uy = 0.f;
+    if (valid)
+    {
+        const float *sn = F.L.snap + at;
+        drho = sn[0];
+        ux = sn[F.L.plane];
+        uy = sn[2 * F.L.plane];
+    }
+    float acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+    {
+        const float w = m[(2 + k) * 32 + lane];
+#pragma unroll
+        for (int q = 0; q < 9; q++)
+        {
+            const float z = __shfl_sync(0xffffffffu, k < 4 ? za[q] : zb[q], base + (k & 3));
+            acc[q] += w * z;
+        }
+    }
+    if (!valid) return;
+    float feq[9];
+    equilibrium(drho, C.rho0 + drho, ux, uy, feq);
+    const float rat = m[8 * 32 + lane];
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+    {
+        acc[q] = feq[q] + rat * (acc[q] - feq[q]);
+        C.ibuf[(size_t)q * C.n_buf + (buf & ~kCoopBuf)] = acc[q];
+    }
+    if (buf & kCoopBuf) CoopSlots(F.L, F.stride, at, F.par).fill(acc);
+}
+
+// fills the block's shared memory (BACK false), or writes the stored |u| back
+template <bool BACK, bool RES>
+__device__ __forceinline__ void coop_cells(const CoopLaunch &A, const CoopRange *rng, float *sm)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int d = 0; d < A.nd; d++)
+    {
+        const CoopDesc &D = A.d[d];
+        for (int kind = 0; kind < CK_KINDS; kind++)
+        {
+            const CoopRange r = rng[d * CK_KINDS + kind];
+            for (int i = warp; i < r.n; i += nw)
+            {
+                const int c = r.lo + i * 32 + lane;
+                const bool there = i * 32 + lane < r.cells;
+                float *m = sm + (size_t)(r.line + i * D.lines[kind]) * 32;
+                float *un = m + (kind >= CK_EDGE ? 2 : 8) * 32 + lane;
+                int xy = -1;
+                if (kind >= CK_EDGE)
+                {
+                    if (there) xy = __ldg(&D.xy[kind][c]);
+                    if (!BACK)
+                    {
+                        const uint32_t site = there ? coop_site(D.L, xy & 0xFFFF, xy >> 16) : kCoopNone;
+                        m[lane] = __uint_as_float(site);
+                        if (there) m[32 + lane] = D.L.omega[site & kCoopSite];
+                    }
+                }
+                else if (there)
+                {
+                    const uint4 *rec = reinterpret_cast<const uint4 *>(D.C.specials + D.spec_begin +
+                                                                       (kind == CK_LIGHT ? D.nheavy : 0) + c);
+                    const uint4 r0 = rec[0], r1 = rec[1];
+                    xy = (int)r1.z;
+                    if (!BACK)
+                    {
+                        reinterpret_cast<uint4 *>(m)[lane] = r0;
+                        reinterpret_cast<uint4 *>(m)[32 + lane] = r1;
+                    }
+                }
+                if (!there || !RES) continue;
+                float *g = &D.L.unorm[site_of(D.L, xy & 0xFFFF, xy >> 16)];
+                if (BACK) *g = *un;
+                else *un = *g;
+            }
+        }
+    }
+}
+
+// DEF: every image has the default regularized MRT and SRBB walls (their code
+// alone then passes through the instruction cache); RES: with residuals (A.every)
+template <int THREADS, bool DEF, bool RES>
+__global__ void __launch_bounds__(THREADS, 1) k_coop_steps(const __grid_constant__ CoopLaunch A)
+{
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ CoopRange rng[kMaxCoopDescs * CK_KINDS], rows[kMaxCoopPairs * 2]; // coarse, fine rows
+    __shared__ uint2 strides[kMaxCoopDescs]; // floats per plane and per row
+    __shared__ unsigned int s_next;          // next unclaimed item of a stage
+    __shared__ double2 s_sums[32];           // the warps' residual terms
+    // this thread's residual terms (in shared memory: registers are what limits the
+    // warps of an SM), then the lines
+    double2 *acc = reinterpret_cast<double2 *>(sm_raw) + threadIdx.x;
+    float *sm = reinterpret_cast<float *>(sm_raw + (RES ? THREADS * sizeof(double2) : 0));
+    const int b = (int)blockIdx.x, G = (int)gridDim.x;
+    for (int t = (int)threadIdx.x; t < A.nd * CK_KINDS; t += (int)blockDim.x)
+    {
+        const int32_t *cut = A.d[t / CK_KINDS].cut[t % CK_KINDS];
+        rng[t].lo = cut[b];
+        rng[t].cells = cut[b + 1] - rng[t].lo;
+        rng[t].n = (rng[t].cells + 31) / 32;
+    }
+    for (int t = (int)threadIdx.x; t < A.nd; t += (int)blockDim.x)
+        strides[t] = make_uint2((uint32_t)A.d[t].L.plane, (uint32_t)A.d[t].L.pitch);
+    for (int t = (int)threadIdx.x; t < A.np * 2; t += (int)blockDim.x)
+    {
+        const CoopPair &Q = A.p[t / 2];
+        const int W = ((t & 1 ? Q.nfine : Q.ncoarse) + 7) / 8;
+        rows[t].lo = coop_cut(W, Q.rot, b, G);
+        rows[t].n = coop_cut(W, Q.rot, b + 1, G) - rows[t].lo;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        s_next = 0u;
+        int line = 0;
+        for (int t = 0; t < A.nd * CK_KINDS; t++)
+        {
+            rng[t].line = line;
+            line += rng[t].n * A.d[t / CK_KINDS].lines[t % CK_KINDS];
+        }
+        for (int t = 0; t < A.np * 2; t++)
+        {
+            rows[t].line = line;
+            line += rows[t].n * (t & 1 ? kCoopFineLines : kCoopCoarseLines);
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    coop_cells<false, RES>(A, rng, sm);
+    for (int t = 0; t < A.np * 2; t++)
+    {
+        const CoopPair &Q = A.p[t / 2];
+        const LevelView &Lf = A.d[Q.df].L, &Lc = A.d[Q.dc].L;
+        for (int i = warp; i < rows[t].n; i += nw)
+        {
+            const int r = (rows[t].lo + i) * 8 + lane / 4;
+            if (t & 1) coop_fill_fine(Q, Lf, Lc, r, lane & 3, sm + (size_t)(rows[t].line + i * kCoopFineLines) * 32);
+            else coop_fill_coarse(Q, Lf, Lc, r, lane & 3, sm + (size_t)(rows[t].line + i * kCoopCoarseLines) * 32);
+        }
+    }
+    __syncthreads();
+    unsigned int target = 0;
+    int since = A.since0, prev = since == 0 ? A.every - 1 : since - 1;
+#pragma unroll 1
+    for (int k = 0; k < A.nsteps; k++)
+    {
+        const bool store = RES && since == 0; // this step's number is a multiple of A.every
+        const bool diff = RES && prev == 0 && !(k == 0 && A.skip_first);
+        if (RES)
+        {
+            prev = since;
+            since = since + 1 == A.every ? 0 : since + 1;
+        }
+#pragma unroll 1
+        for (int ph = 0; ph < A.nphase; ph++)
+        {
+            CoopClaim claim(&s_next);
+            if (RES && diff && ph == 0) *acc = make_double2(0.0, 0.0);
+#pragma unroll 1
+            for (int d = 0; d < A.nd; d++)
+            {
+                const CoopDesc &D = A.d[d];
+                if (ph & ((1 << D.shift) - 1)) continue;
+                const int sub = ph >> D.shift;
+                CoopStep st{};
+                st.o.parity = (D.parity0 + k * D.substeps + sub) & 1;
+                st.o.direct = k == 0 && sub == 0 && D.direct0;
+                st.o.first_sub = sub == 0;
+                st.o.snap_store = D.mb && sub == 0;
+                st.o.snap_use = D.mb && sub > 0;
+                st.diff = diff && sub == 0;
+                st.store_u = store && sub == 0;
+                st.collision = DEF ? COLL_RMRT : D.C.collision;
+                st.wall = DEF ? WALL_SRBB : D.C.wall;
+                coop_level<RES>(A, d, st, rng + d * CK_KINDS, strides + d, sm, claim, acc);
+            }
+            if (RES && diff && ph == 0) block_sums(acc->x, acc->y, s_sums);
+            const bool end = k + 1 == A.nsteps && ph + 1 == A.nphase && A.nwave == 0;
+            if (RES && diff && ph == 0)
+            {
+                double *red = A.d[0].C.red + (size_t)((uint32_t)(A.slot0 + k) % (uint32_t)A.ring) * 4;
+                if (!end)
+                {
+                    target += gridDim.x;
+                    if (!grid_barrier(A.bar, target, A.err, nullptr, nullptr, &s_next, s_sums, red)) return;
+                    continue;
+                }
+                __syncthreads();
+                if (warp == 1) add_block_sums(s_sums, red);
+            }
+            if (end) break;
+            target += gridDim.x;
+            if (!grid_barrier(A.bar, target, A.err, nullptr, nullptr, &s_next)) return;
+        }
+#pragma unroll 1
+        for (int w = 0; w < A.nwave; w++)
+        {
+            CoopClaim claim(&s_next);
+#pragma unroll 1
+            for (int p = 0; p < A.np; p++)
+            {
+                const CoopPair &Q = A.p[p];
+                const int kind = Q.l1 - 1 == w ? 0 : Q.l1 == w ? 1 : -1; // coarse rows / fine rows
+                if (kind < 0) continue;
+                const CoopRange rr = rows[p * 2 + kind];
+                const int nrows = kind == 0 ? Q.ncoarse : Q.nfine;
+                const CoopDesc &F = A.d[Q.df], &Cd = A.d[Q.dc];
+                const int pf = (F.parity0 + (k + 1) * F.substeps) & 1, pc = (Cd.parity0 + (k + 1) * Cd.substeps) & 1;
+                const CoopSide fine{F.L, strides + Q.df, pf}, coarse{Cd.L, strides + Q.dc, pc};
+#pragma unroll 1
+                for (int i; (i = claim.mine - claim.base) < rr.n; claim.claim())
+                {
+                    const int r = (rr.lo + i) * 8 + lane / 4;
+                    const bool valid = r < nrows;
+                    const float *m = sm + (size_t)(rr.line + i * (kind == 0 ? kCoopCoarseLines : kCoopFineLines)) * 32;
+                    const bool slow = __any_sync(0xffffffffu, __float_as_int(m[(kind == 0 ? 2 : 11) * 32 + lane]) != 0);
+                    if (kind == 0)
+                    {
+                        const CoarseRowDev &row = Q.coarse[valid ? r : 0];
+                        if (!slow) coop_coarse(fine, coarse, F.C, m, valid);
+                        else if (pf) coarse_row<1>(F.L, Cd.L, F.C, row, lane & 3, valid, pc);
+                        else coarse_row<0>(F.L, Cd.L, F.C, row, lane & 3, valid, pc);
+                    }
+                    else
+                    {
+                        const FineRowDev &row = Q.fine[valid ? r : 0];
+                        if (!slow) coop_fine(fine, coarse, F.C, m, valid);
+                        else if (pc) fine_child<1>(F.L, Cd.L, F.C, row, lane & 3, valid, pf);
+                        else fine_child<0>(F.L, Cd.L, F.C, row, lane & 3, valid, pf);
+                    }
+                }
+                claim.base += rr.n;
+            }
+            if (k + 1 == A.nsteps && w + 1 == A.nwave) break;
+            target += gridDim.x;
+            if (!grid_barrier(A.bar, target, A.err, nullptr, nullptr, &s_next)) return;
+        }
+    }
+    if (RES)
+    {
+        __syncthreads(); // the last stage has no barrier: other warps' |u| are still being stored
+        coop_cells<true, RES>(A, rng, sm);
     }
 }
 

@@ -24,11 +24,6 @@ inline bool special_is_light(const SpecialRec &r)
     return !wall && !over && !quirk && !(flags & (SF_INLET | SF_OUTLET));
 }
 
-inline uint64_t special_order_key(int32_t xy)
-{
-    const uint64_t x = (uint64_t)(xy & 0xFFFF), y = (uint64_t)((uint32_t)xy >> 16);
-    return ((y >> 2) << 40) | ((x >> 3) << 20) | ((y & 3) << 8) | (x & 7);
-}
 } // namespace
 
 namespace
@@ -283,24 +278,18 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
         L.specials.push_back(rec);
         spec_level.push_back(l);
     }
-    // special records grouped by level, heavy before light, then by whether they
-    // have wall links, then ordered by 8x4 block of sites (row-major blocks,
-    // row-major inside a block), so a warp of the special-cell kernel takes one
-    // path over a compact patch
+    // special records grouped by level, heavy before light, then ordered by place
+    // (site_order_key), so a warp of them covers a compact patch
     {
         std::vector<int64_t> order(L.specials.size());
         for (size_t i = 0; i < order.size(); i++) order[i] = (int64_t)i;
-        std::sort(order.begin(), order.end(), [&](int64_t a, int64_t b) {
-            if (spec_level[a] != spec_level[b]) return spec_level[a] < spec_level[b];
-            // heavy records first, light ones last (the 8x4 plain kernel can take
-            // those); cells with wall links apart from the others, so the warps of
-            // the special-cell kernel take one path
-            const bool la = special_is_light(L.specials[a]), lb = special_is_light(L.specials[b]);
-            if (la != lb) return la < lb;
-            const bool wa = ((L.specials[a].m0 >> 18) & 0x1FFu) != 0, wb = ((L.specials[b].m0 >> 18) & 0x1FFu) != 0;
-            if (wa != wb) return wa < wb;
-            return special_order_key(L.specials[a].xy) < special_order_key(L.specials[b].xy);
-        });
+        // key: level, heavy records first and light ones last (the 8x4 plain kernel
+        // can take those), place
+        std::vector<uint64_t> key(order.size());
+        for (size_t i = 0; i < order.size(); i++)
+            key[i] = (uint64_t)spec_level[i] << 33 | (uint64_t)special_is_light(L.specials[i]) << 32 |
+                     site_order_key(L.specials[i].xy);
+        std::sort(order.begin(), order.end(), [&](int64_t a, int64_t b) { return key[(size_t)a] < key[(size_t)b]; });
         std::vector<SpecialRec> sorted(order.size());
         for (size_t i = 0; i < order.size(); i++) sorted[i] = L.specials[order[i]];
         L.specials.swap(sorted);
@@ -357,13 +346,26 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
         }
     }
 
-    // plain cells in row order, for the adsorption engine that gives each thread
-    // its cells for many steps
-    if (p.adsorption)
-        for (auto &lv : L.levels)
+    // plain cells for the engines that give each thread its cells for many steps:
+    // those that are no buffer cells, then the buffer cells, each ordered by place
+    for (auto &lv : L.levels)
+    {
+        std::vector<char> is_buf((size_t)lv.plane, 0);
+        for (size_t i = 0; i < L.buf_level.size(); i++)
+            if (L.buf_level[i] == lv.level) is_buf[(size_t)L.buf_site[i]] = 1;
+        for (int kind = 0; kind < 2; kind++)
+        {
+            const size_t begin = lv.plain_xy.size();
             for (int y = 0; y < lv.H; y++)
                 for (int x = 0; x < lv.W; x++)
-                    if (lv.omega[(size_t)y * lv.pitch + x] > 0.0f) lv.plain_xy.push_back(x | y << 16);
+                {
+                    const size_t s = (size_t)y * lv.pitch + x;
+                    if (!(lv.omega[s] > 0.0f)) continue;
+                    if (is_buf[s] == kind) lv.plain_xy.push_back(x | y << 16);
+                }
+            lv.n_plain[kind] = (int64_t)(lv.plain_xy.size() - begin);
+        }
+    }
 
     // 8x4 tiles holding a plain or light cell, row-major (one warp per tile in the
     // 8x4 kernel: sparse levels fill them better than 32x8 tiles), with the mask
@@ -442,6 +444,8 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
             d.ratio = (float)(2 * g.tau[row[0]] / (tsum / cnt));
             d.inv_nchild = 1.0f / cnt;
             d.plain_target = plain_buffer[row[0]];
+            for (int k = 0; k < 4; k++)
+                if (d.child[k] >= 0 && d.child_buf[k] < 0 && L.levels[l1 - 1].omega[(size_t)d.child[k]] < 0.0f) d.special = 1;
             itf.coarse.push_back(d);
         }
         const int top_order[9] = {7, 4, 8, 3, 0, 1, 6, 2, 5};
@@ -493,6 +497,7 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
                 int64_t src = nb >= 0 ? nb : pc;
                 d.node_site[k] = L.cell_site[src];
                 d.node_buf[k] = (is_coarse_buffer(src) && g.level[src] <= l2) ? buf_of[src] : -1;
+                if (d.node_buf[k] < 0 && L.levels[l2 - 1].omega[(size_t)d.node_site[k]] < 0.0f) d.special = 1;
             }
             for (int k = 0; k < 4; k++)
             {
@@ -513,6 +518,13 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
             }
             itf.fine.push_back(d);
         }
+        // rows ordered by the place of their (first) target: sites are row-major
+        auto by_coarse = [](const CoarseRowDev &a, const CoarseRowDev &b) { return a.site < b.site; };
+        auto by_fine = [](const FineRowDev &a, const FineRowDev &b) { return a.child_site[0] < b.child_site[0]; };
+        if (!std::is_sorted(itf.coarse.begin(), itf.coarse.end(), by_coarse))
+            std::sort(itf.coarse.begin(), itf.coarse.end(), by_coarse);
+        if (!std::is_sorted(itf.fine.begin(), itf.fine.end(), by_fine))
+            std::sort(itf.fine.begin(), itf.fine.end(), by_fine);
         L.interfaces.push_back(std::move(itf));
     }
 
@@ -535,5 +547,41 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
     }
     L.tau_mean = nt ? ts / nt : 0.0;
     return L;
+}
+
+// Equal shares of a level's cells: lists sorted by site_order_key, cut where the
+// weight of all cells before the key reaches k / parts of the total.
+std::vector<std::vector<int32_t>> share_cuts(const std::vector<ShareList> &lists, int parts)
+{
+    double total = 0;
+    for (const ShareList &l : lists) total += l.weight * (double)l.n;
+    std::vector<std::vector<int32_t>> cuts(lists.size(), std::vector<int32_t>((size_t)parts + 1, 0));
+    std::vector<int32_t> at(lists.size(), 0);
+    double done = 0;
+    for (int k = 1; k <= parts; k++)
+    {
+        const double goal = total * k / parts;
+        while (k == parts || done < goal)
+        {
+            // the list whose next cell comes first
+            int best = -1;
+            uint32_t key = 0;
+            for (size_t l = 0; l < lists.size(); l++)
+            {
+                if (at[l] >= lists[l].n) continue;
+                const uint32_t kl = site_order_key(lists[l].xy[(size_t)at[l] * lists[l].stride]);
+                if (best < 0 || kl < key)
+                {
+                    best = (int)l;
+                    key = kl;
+                }
+            }
+            if (best < 0) break;
+            at[(size_t)best]++;
+            done += lists[(size_t)best].weight;
+        }
+        for (size_t l = 0; l < lists.size(); l++) cuts[l][(size_t)k] = at[l];
+    }
+    return cuts;
 }
 } // namespace mantiis

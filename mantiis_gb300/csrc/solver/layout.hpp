@@ -79,7 +79,9 @@ struct LevelLayout
     std::vector<int32_t> tile8_list;  // 8x4 tiles holding a plain or light cell: tx | ty << 16 (x in 8s, y in 4s)
     std::vector<uint32_t> tile8_mask; // per such tile, its plain and light cells (bit = 8 * row + column)
     std::vector<uint32_t> tile8_light;// per such tile, its light cells (subset of tile8_mask)
-    std::vector<int32_t> plain_xy;    // plain cells, row-major: x | y << 16 (adsorption only)
+    std::vector<int32_t> plain_xy;    // plain cells, x | y << 16: those that are no buffer cells, then the buffer
+                                      // cells, each ordered by place
+    int64_t n_plain[2] = {0, 0};      // how many of each
     int64_t n_active = 0, n_active_real = 0;
     int substeps = 1;                // per coarse step, 2^(L-l)
     int64_t spec_begin = 0, spec_count = 0; // this level's special records (sorted by site)
@@ -100,7 +102,8 @@ struct CoarseRowDev
     float ratio;         // 2 tau_c / mean(tau_children)
     float inv_nchild;    // 1 / number of children present
     int32_t plain_target;// the coarse cell steps as a plain cell: its values also go to the slots it reads next
-    int32_t pad_[3];     // 64 bytes: rows stay 16-byte aligned in an array
+    int32_t special;     // some child is a special cell
+    int32_t pad_[2];     // 64 bytes: rows stay 16-byte aligned in an array
 };
 static_assert(sizeof(CoarseRowDev) % 16 == 0, "coarse row size");
 
@@ -114,7 +117,8 @@ struct FineRowDev
     float weight[4][6];  // interpolation weights per child
     float ratio[4];      // tau_child / (2 tau_parent)
     int32_t plain_mask;  // bit c: child c steps as a plain cell (values also go to the slots it reads next)
-    int32_t pad_[3];
+    int32_t special;     // some node not in the interpolation buffer is a special cell
+    int32_t pad_[2];
 };
 static_assert(sizeof(FineRowDev) % 16 == 0, "fine row size");
 
@@ -153,6 +157,24 @@ struct ImageLayout
 };
 
 ImageLayout build_layout(const Grid &g, const LayoutParams &p);
+
+// Order of cells by place: row by row.  A contiguous share of such a list is a band
+// of the level, whatever the kind of cell, so the cells of one SM read each
+// other's sectors; long rows keep a warp's cells side by side (us per step of the
+// cooperative engine at 1024^2, single block / two levels, with the cells in
+// 32x32 tiles along a Z curve 13.6 / 39, 128x16 12.5 / 36, in rows 12.5 / 34).
+inline uint32_t site_order_key(int32_t xy) { return (uint32_t)xy; } // x | y << 16
+
+// one list of cells sorted by site_order_key: x | y << 16 of cell i at xy[i * stride]
+struct ShareList
+{
+    const int32_t *xy;
+    int32_t n;
+    int stride;
+    double weight; // work of a cell
+};
+// per list the parts + 1 cuts that give every part the same work and the same patch
+std::vector<std::vector<int32_t>> share_cuts(const std::vector<ShareList> &lists, int parts);
 
 // Interpolation weights of the reference's fine-buffer bicubic spline for one
 // parent (exposed for tests): nodes x[3], y[2] and the query points (qx, qy),

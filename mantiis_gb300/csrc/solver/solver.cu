@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -112,6 +113,10 @@ struct LevelDev
     DevBuf<float> f, omega, tau2, snap, unorm, psi, rho_prev;
     DevBuf<uint32_t> spec;
     DevBuf<int32_t> tiles, tiles8, plain_xy;
+    // shares of the level's cells per SM, by kind (dev::CoopKind): sm_count + 1
+    // cuts each
+    DevBuf<int32_t> cuts;
+    std::vector<int32_t> cuts_host;
     DevBuf<uint32_t> tile_mask, tile8_mask, tile8_light;
     int64_t steps = 0; // substeps done at this level
 };
@@ -160,6 +165,21 @@ struct PersistPlan
     int nseg = 0, total_units = 0, nctr = 0;
     int tiles_per_warp = 1;
     int64_t bytes = 0;
+};
+
+// Cooperative launch of a group of transport images (dev::k_coop_steps): its
+// parameters but for the state of the levels, and its shape.
+struct CoopPlan
+{
+    std::vector<mgpu_ctx *> ctxs;
+    dev::CoopLaunch L;
+    int grid = 0;
+    int threads[2] = {0, 0}; // without / with residuals
+    size_t smem[2] = {0, 0};
+    bool def = true; // default collision and walls in every image
+    const void *kernel[2] = {nullptr, nullptr};
+    bool ok = false; // the group fits the kernel's tables and shared memory
+    bool ok_residual = false; // with residuals too
 };
 
 } // namespace
@@ -250,11 +270,13 @@ struct mgpu_ctx
     DevBuf<double> out_rho, out_ux, out_uy, out_f;
     DevBuf<double> in_rho, in_ux, in_uy; // staging of mgpu_set_equilibrium, kept between calls
     DevBuf<unsigned int> errword;
-    // adsorption step engine: MGPU_ENGINE_PERSISTENT runs many steps in one
-    // cooperative launch (k_ads_persistent), MGPU_ENGINE_STREAMS launches the
-    // passes (pairs of steps replayed from a CUDA graph)
+    // step engine: MGPU_ENGINE_PERSISTENT runs many steps in one cooperative
+    // launch (k_ads_persistent; transport contexts that qualify, coop_ok:
+    // k_coop_steps), MGPU_ENGINE_STREAMS launches the passes or phases (pairs of
+    // steps replayed from a CUDA graph)
     int engine = MGPU_ENGINE_PERSISTENT;
-    DevBuf<unsigned int> ads_bar; // grid-barrier arrivals of k_ads_persistent
+    DevBuf<unsigned int> grid_bar; // grid-barrier arrivals of the cooperative launches
+    std::unique_ptr<CoopPlan> coop; // cooperative transport launch of this image
     float rho0f = 0.f;
     bool adsorption = false; // Shan-Chen step body (include/mantiisApp.hpp:248-265)
     // coupled run (include/mantiisApp.hpp:376-392): up to 100 adsorption steps
@@ -812,7 +834,7 @@ void run_ads_persistent(mgpu_ctx *ctx, int n, int64_t k, bool diff)
     A.slot0 = (int)(k % kRing);
     A.ring = kRing;
     A.psi_diff = diff ? 1 : 0; // the density change (the coupling phase, with |u| sums, is not run here)
-    A.bar = ctx->ads_bar.p;
+    A.bar = ctx->grid_bar.p;
     // one block per SM with at least four warps of cells each; the warps of a
     // block share its warps of cells evenly, as much of their data as fits in
     // shared memory
@@ -847,6 +869,164 @@ void run_ads_persistent(mgpu_ctx *ctx, int n, int64_t k, bool diff)
     ctx->launches++;
     ctx->lv[0].steps += n;
     ctx->coarse_done += n;
+}
+
+// ---- cooperative transport steps, host side
+// most threads of a block (80 registers each; 512 and 1024 threads measured slower
+// at 1024^2, single block: 15.1 and 13.9 against 13.6 us per step)
+constexpr int kCoopThreads = 768;
+constexpr int kCoopResThreads = 640; // with residuals (96 registers: nothing spilled)
+
+std::unique_ptr<CoopPlan> build_coop(const std::vector<mgpu_ctx *> &ctxs)
+{
+    std::unique_ptr<CoopPlan> P(new CoopPlan());
+    P->ctxs = ctxs;
+    std::memset(&P->L, 0, sizeof(P->L));
+    dev::CoopLaunch &A = P->L;
+    const int G = ctxs[0]->sm_count;
+    int Lmax = 1;
+    for (auto *c : ctxs) Lmax = std::max(Lmax, c->lay.max_level);
+    A.nphase = 1 << (Lmax - 1);
+    A.nwave = Lmax >= 2 ? Lmax : 0;
+    A.ring = kRing;
+    for (auto *c : ctxs)
+    {
+        const int base = A.nd, L = c->lay.max_level;
+        if (A.nd + L > dev::kMaxCoopDescs || A.np + (int)c->itf.size() > dev::kMaxCoopPairs) return P;
+        for (int l = 0; l < L; l++)
+        {
+            const LevelLayout &ll = c->lay.levels[l];
+            if (ll.plane > (int64_t)dev::kCoopSite) return P; // sites in 28 bits, slots in 32
+            dev::CoopDesc &D = A.d[A.nd++];
+            D.L = c->view(l);
+            D.C = c->common();
+            D.spec_begin = ll.spec_begin;
+            D.nheavy = (int)ll.spec_heavy;
+            D.xy[dev::CK_PLAIN] = c->lv[l].plain_xy.p;
+            D.xy[dev::CK_EDGE] = D.xy[dev::CK_PLAIN] + ll.n_plain[0];
+            for (int k = 0; k < dev::CK_KINDS; k++) D.cut[k] = c->lv[l].cuts.p + (size_t)k * (G + 1);
+            D.lines[dev::CK_HEAVY] = D.lines[dev::CK_LIGHT] = dev::kCoopRecLines;
+            D.lines[dev::CK_EDGE] = dev::kCoopPlainLines;
+            D.lines[dev::CK_PLAIN] = dev::kCoopPlainLines + (ll.substeps > 1 ? dev::kCoopSnapLines : 0);
+            P->def = P->def && c->prm.collision == COLL_RMRT && c->prm.wall == WALL_SRBB;
+            D.shift = Lmax - L + l;
+            D.substeps = ll.substeps;
+            D.mb = c->grid.multiblock ? 1 : 0;
+        }
+        for (const InterfaceDev &it : c->itf)
+        {
+            dev::CoopPair &Q = A.p[A.np];
+            Q.coarse = it.coarse.p;
+            Q.fine = it.fine.p;
+            Q.ncoarse = it.ncoarse;
+            Q.nfine = it.nfine;
+            Q.df = base + it.l1 - 1;
+            Q.dc = base + it.l1;
+            Q.l1 = it.l1;
+            Q.rot = (A.np++ * 61) % G;
+        }
+    }
+    // shared memory and warps of cells of the fullest block; in phase 0 every
+    // level steps
+    int64_t lines = 0;
+    int warps = 1;
+    for (int b = 0; b < G; b++)
+    {
+        int64_t ln = 0;
+        int w = 0;
+        int d = 0;
+        for (auto *c : ctxs)
+            for (const LevelDev &lv : c->lv)
+            {
+                for (int k = 0; k < dev::CK_KINDS; k++)
+                {
+                    const int32_t *cut = &lv.cuts_host[(size_t)k * (G + 1) + b];
+                    const int n = (cut[1] - cut[0] + 31) / 32;
+                    ln += (int64_t)n * A.d[d].lines[k];
+                    w += n;
+                }
+                d++;
+            }
+        for (int p = 0; p < A.np; p++)
+            for (int k = 0; k < 2; k++)
+            {
+                const int W = ((k ? A.p[p].nfine : A.p[p].ncoarse) + 7) / 8, rot = A.p[p].rot;
+                ln += (int64_t)(dev::coop_cut(W, rot, b + 1, G) - dev::coop_cut(W, rot, b, G)) *
+                      (k ? dev::kCoopFineLines : dev::kCoopCoarseLines);
+            }
+        lines = std::max(lines, ln);
+        warps = std::max(warps, w);
+    }
+    int smem_max = 0;
+    CK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctxs[0]->device));
+    const size_t room = (size_t)smem_max - 5120; // (the kernel's static shared memory)
+    P->smem[0] = (size_t)lines * 128;
+    P->smem[1] = P->smem[0] + (size_t)kCoopResThreads * sizeof(double2); // the threads' residual terms
+    if (P->smem[0] > room) return P;
+    P->ok_residual = P->smem[1] <= room;
+    P->grid = G;
+    for (int res = 0; res < 2; res++)
+    {
+        const int most = (res ? kCoopResThreads : kCoopThreads) / 32, rounds = (warps + most - 1) / most;
+        P->threads[res] = std::max(4, (warps + rounds - 1) / rounds) * 32;
+    }
+    P->kernel[0] = P->def ? (const void *)dev::k_coop_steps<kCoopThreads, true, false>
+                          : (const void *)dev::k_coop_steps<kCoopThreads, false, false>;
+    P->kernel[1] = P->def ? (const void *)dev::k_coop_steps<kCoopResThreads, true, true>
+                          : (const void *)dev::k_coop_steps<kCoopResThreads, false, true>;
+    for (const void *k : P->kernel) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    P->ok = true;
+    return P;
+}
+
+// n coarse steps of the plan's images in one launch on `st`.  every > 0 (one
+// image): residuals as dev::CoopLaunch describes, into zeroed slots.
+void run_coop(CoopPlan &P, int n, int every, bool skip_first, unsigned int *bar, cudaStream_t st, int64_t &launches)
+{
+    dev::CoopLaunch &A = P.L;
+    // a launch holds every SM: other streams' kernels get their turn between
+    // launches (the fill of shared memory at its start takes about 10 us)
+    constexpr int kMaxSteps = 500;
+    for (int done = 0; done < n;)
+    {
+        A.nsteps = std::min(kMaxSteps, n - done);
+        A.every = every;
+        // (the state before the first step of all has no stored |u|)
+        A.skip_first = (skip_first && done == 0) || P.ctxs[0]->coarse_done == 0 ? 1 : 0;
+        const int64_t k0 = P.ctxs[0]->coarse_done + 1; // the launch's first step
+        A.since0 = every ? (int)(k0 % every) : 0;
+        A.slot0 = (int)((k0 - 1) % kRing);
+        A.bar = bar;
+        A.err = P.ctxs[0]->errword.p;
+        int d = 0;
+        for (auto *c : P.ctxs)
+            for (auto &l : c->lv)
+            {
+                A.d[d].parity0 = (int)(l.steps & 1);
+                A.d[d++].direct0 = l.steps == 0 ? 1 : 0;
+            }
+        CK(cudaMemsetAsync(bar, 0, sizeof(unsigned int), st));
+        void *args[] = {&A};
+        CK(cudaLaunchCooperativeKernel(P.kernel[every > 0], dim3((unsigned)P.grid), dim3((unsigned)P.threads[every > 0]), args, P.smem[every > 0], st));
+        launches++;
+        for (auto *c : P.ctxs)
+        {
+            for (size_t l = 0; l < c->lv.size(); l++) c->lv[l].steps += (int64_t)A.nsteps * c->lay.levels[l].substeps;
+            c->coarse_done += A.nsteps;
+        }
+        done += A.nsteps;
+    }
+}
+
+// A transport context steps by cooperative launches unless the caller chose a
+// plain-cell kernel (plain_path), the launch engine, or said that other contexts
+// share the GPU.
+bool coop_ok(mgpu_ctx *ctx, bool residual)
+{
+    if (ctx->adsorption || ctx->engine != MGPU_ENGINE_PERSISTENT || ctx->prm.plain_path >= 0 || ctx->prm.concurrent)
+        return false;
+    if (!ctx->coop) ctx->coop = build_coop({ctx});
+    return residual ? ctx->coop->ok_residual : ctx->coop->ok;
 }
 
 bool fresh_state(const mgpu_ctx *ctx)
@@ -890,6 +1070,9 @@ void run_batch_with_residuals(mgpu_ctx *ctx, int n)
         }
         return;
     }
+    if (n > 0 && coop_ok(ctx, true))
+        run_coop(*ctx->coop, n, 1, true, ctx->grid_bar.p, ctx->stream, ctx->launches);
+    else
     for (int i = 0; i < n;)
     {
         int64_t k = ctx->coarse_done + 1; // this step
@@ -1563,6 +1746,21 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
         d.tile_mask.upload(ll.tile_mask, acct, s);
         d.tiles8.upload(ll.tile8_list, acct, s);
         d.plain_xy.upload(ll.plain_xy, acct, s);
+        if (!ctx->adsorption)
+        {
+            const int32_t *rec = reinterpret_cast<const int32_t *>(ctx->lay.specials.data() + ll.spec_begin) +
+                                 offsetof(SpecialRec, xy) / sizeof(int32_t);
+            constexpr int rs = sizeof(SpecialRec) / sizeof(int32_t);
+            const int32_t *xy = ll.plain_xy.data();
+            std::vector<ShareList> lists(dev::CK_KINDS);
+            // weights: the time of a cell of each kind, in plain cells
+            lists[dev::CK_HEAVY] = {rec, (int32_t)ll.spec_heavy, rs, 3.0};
+            lists[dev::CK_LIGHT] = {rec + rs * ll.spec_heavy, (int32_t)(ll.spec_count - ll.spec_heavy), rs, 1.5};
+            lists[dev::CK_PLAIN] = {xy, (int32_t)ll.n_plain[0], 1, 1.0};
+            lists[dev::CK_EDGE] = {xy + ll.n_plain[0], (int32_t)ll.n_plain[1], 1, 1.0};
+            for (const auto &c : share_cuts(lists, ctx->sm_count)) d.cuts_host.insert(d.cuts_host.end(), c.begin(), c.end());
+            d.cuts.upload(d.cuts_host, acct, s);
+        }
         d.tile8_mask.upload(ll.tile8_mask, acct, s);
         d.tile8_light.upload(ll.tile8_light, acct, s);
         d.use8 = p->plain_path == 2 && !ctx->adsorption;
@@ -1605,7 +1803,7 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
     ctx->red.zero(s);
     ctx->errword.alloc(1, acct);
     ctx->errword.zero(s);
-    if (ctx->adsorption) ctx->ads_bar.alloc(1, acct);
+    ctx->grid_bar.alloc(1, acct);
     for (auto &it : ctx->lay.interfaces)
     {
         ctx->itf.emplace_back();
@@ -1828,6 +2026,18 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
                 if ((int)pending.size() >= kRing / 2) flush();
                 continue;
             }
+            if (coop_ok(ctx, true))
+            {
+                // the rest of the call (as many steps as the pending slots hold) in one launch
+                const int m = std::min(n_steps - i, kRing / 2 - (int)pending.size());
+                zero_slots(ctx, (int)((k - 1) % kRing), m);
+                run_coop(*ctx->coop, m, K, false, ctx->grid_bar.p, ctx->stream, ctx->launches);
+                for (int64_t j = k; j < k + m; j++)
+                    if (j >= 2 && (j - 1) % K == 0) pending.push_back(j - 1);
+                i += m - 1;
+                if ((int)pending.size() >= kRing / 2) flush();
+                continue;
+            }
             // residual of step s is evaluated by kernel s+1 against |u| stored by kernel s
             bool diff = k >= 2 && ((k - 1) % K == 0);
             bool store = (k % K == 0);
@@ -1861,6 +2071,12 @@ int mgpu_advance_graph(mgpu_ctx *ctx, int n_steps)
         if (ads_persistent_ok(ctx))
         {
             if (n_steps > 0) run_ads_persistent(ctx, n_steps, ctx->coarse_done + 1, false);
+            ctx->ref_t += n_steps;
+            return MGPU_OK;
+        }
+        if (coop_ok(ctx, false))
+        {
+            run_coop(*ctx->coop, n_steps, 0, false, ctx->grid_bar.p, ctx->stream, ctx->launches);
             ctx->ref_t += n_steps;
             return MGPU_OK;
         }
@@ -2380,6 +2596,10 @@ struct mgpu_batch
     // batch of 4 at 5 blocks per SM: 4 -> 408 us per coarse step, 2 -> 443, 1 -> 459;
     // at 4 blocks per SM 436, at 3 630)
     int engine = 0, group = 0, tiles_per_warp = 4;
+    // until mgpu_batch_set_engine: groups of images stepped by cooperative
+    // launches where every group fits (else engine 0)
+    bool engine_set = false;
+    std::vector<std::unique_ptr<CoopPlan>> coop;
     std::map<std::string, std::unique_ptr<PersistPlan>> pplans;
     DevBuf<unsigned int> sync; // claim and stage counters of the persistent launch
     int64_t bytes = 0;
@@ -2404,6 +2624,47 @@ void batch_leave(mgpu_batch *b)
     CK(cudaEventRecord(b->ev_done, b->stream));
     for (auto *c : b->ctxs)
         if (c->stream != b->stream) CK(cudaStreamWaitEvent(c->stream, b->ev_done, 0));
+}
+
+// Groups of the batch's images for the cooperative engine, in order: as many
+// together as their state fits twice the L2 (dense planes, of which a step touches
+// the cells' sectors) and the kernel's tables.  us per coarse step of a batch with
+// groups of 1x / 2x / 4x the L2: four 1024^2 images of two levels 137 / 130 / 142
+// (the launch engine: 141), of one level 48 / 44 / 62 (58), six of mixed sizes
+// 84 / 58 / 58 (62).  Images beyond that size keep the launch engine, whose
+// images overlap (two 2048^2 images of two levels: 197, launches 186).
+bool batch_coop(mgpu_batch *b)
+{
+    if (b->coop.empty())
+    {
+        int l2 = 0;
+        CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, b->ctxs[0]->device));
+        const int64_t most = 2 * (int64_t)l2;
+        for (auto *c : b->ctxs)
+            if (c->bytes > most) return false;
+        std::vector<mgpu_ctx *> group;
+        int64_t bytes = 0;
+        std::unique_ptr<CoopPlan> plan;
+        for (auto *c : b->ctxs)
+        {
+            group.push_back(c);
+            bytes += c->bytes;
+            std::unique_ptr<CoopPlan> more = build_coop(group);
+            if (plan && (bytes > most || !more->ok))
+            {
+                // the group ends before this image
+                b->coop.push_back(std::move(plan));
+                group = {c};
+                bytes = c->bytes;
+                more = build_coop(group);
+            }
+            plan = std::move(more);
+        }
+        b->coop.push_back(std::move(plan));
+    }
+    for (auto &g : b->coop)
+        if (!g->ok) return false;
+    return true;
 }
 
 // the persistent plan of the batch's current state for n coarse steps
@@ -2528,6 +2789,13 @@ int mgpu_batch_advance(mgpu_batch *b, int n_steps)
     return guarded(nullptr, [&]() {
         if (!b || n_steps < 0) throw std::invalid_argument("bad argument");
         batch_enter(b);
+        if (!b->engine_set && batch_coop(b))
+        {
+            for (auto &g : b->coop) run_coop(*g, n_steps, 0, false, b->sync.p, b->stream, b->launches);
+            for (auto *c : b->ctxs) c->ref_t += n_steps;
+            batch_leave(b);
+            return MGPU_OK;
+        }
         int left = n_steps;
         // the graph starts from a stepped state (not the initial "direct" one)
         bool fresh = false;
@@ -2684,7 +2952,9 @@ int mgpu_batch_set_engine(mgpu_batch *b, int engine, int group)
 {
     return guarded(nullptr, [&]() {
         if (!b || engine < 0 || engine > 1 || group < 0) throw std::invalid_argument("bad argument");
-        if (engine == b->engine && group == b->group) return MGPU_OK;
+        const bool was_set = b->engine_set;
+        b->engine_set = true;
+        if (was_set && engine == b->engine && group == b->group) return MGPU_OK;
         CK(cudaStreamSynchronize(b->stream));
         if (b->graph)
         {

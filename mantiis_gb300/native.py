@@ -319,8 +319,8 @@ class Solver:
         self._check(lib().mgpu_advance_graph(self._h, int(n_steps)))
 
     def set_engine(self, engine):
-        """Adsorption step engine (mgpu_set_engine): 1 (default) the steps of a
-        call in one cooperative launch, 0 launches per pass."""
+        """Step engine (mgpu_set_engine): 1 (default) the steps of a call in
+        cooperative launches, 0 launches per pass or phase."""
         self._check(lib().mgpu_set_engine(self._h, int(engine)))
 
     def step_level(self, level, n):
@@ -445,8 +445,7 @@ class Solver:
 
 
 class Batch:
-    """Several Solver contexts stepped together (include/mantiis_gpu.h, mgpu_batch):
-    one launch per phase over every image, two coarse steps per CUDA graph."""
+    """Several Solver contexts stepped together (include/mantiis_gpu.h, mgpu_batch)."""
 
     def __init__(self, solvers):
         self._h = None
