@@ -46,11 +46,11 @@ MANTIIS_HD inline bool within_distance(int64_t s, double D)
     return fabs(sqrt((double)s) - D) < 1.0e-4;
 }
 
-// skel: n*n row-major, non-zero on skeleton pixels.  Returns the linear index
+// skel[r * n + c]: non-zero on skeleton pixels.  Returns the linear index
 // r * n + c of the hit, or -1.  D larger than any distance inside the image
 // (no skeleton pixel at all gives the float maximum) returns -1 at once.
-template <typename Pixel>
-MANTIIS_HD inline int64_t nearest_skeleton_at(const Pixel *skel, int n, int i, int j, double D)
+template <typename Skeleton>
+MANTIIS_HD inline int64_t nearest_skeleton_at(const Skeleton &skel, int n, int i, int j, double D)
 {
     const double tol = 1.0e-4;
     if (!(D >= 0.0 && D <= 2.0 * (double)n)) return -1;
@@ -86,6 +86,29 @@ MANTIIS_HD inline int64_t nearest_skeleton_at(const Pixel *skel, int n, int i, i
                 if (c < c0 || !((double)c < c_end) || c < 0 || c >= n) continue;
                 if (skel[r * n + c]) return r * n + c;
             }
+    }
+    return -1;
+}
+
+// The same for D = sqrtf(s) of an exact squared distance 0 <= s <= 10^6: then s
+// alone passes the reference's test.  D is within 6e-8 D <= 6e-5 of sqrt(s), and
+// the square roots of s - 1 and s + 1 are at least 1 / (2 sqrt(s + 1)) > 4.9e-4
+// away from it.  A row can pass at the one column distance m with m^2 = s - di^2,
+// if that is a square, and the window holds every such pixel of the image.
+constexpr int32_t kExactSquares = 1000000;
+template <typename Skeleton>
+MANTIIS_HD inline int64_t nearest_skeleton_at_square(const Skeleton &skel, int n, int i, int j, int32_t s)
+{
+    const int d = (int)sqrtf((float)s); // s < 2^24: exact, and so are the roots of squares below
+    for (int di = i < d ? i : d; di >= -d && i - di < n; di--)
+    {
+        const int32_t b = s - di * di;
+        if (b < 0) continue;
+        const int m = (int)sqrtf((float)b);
+        if (m * m != b) continue;
+        const int64_t row = (int64_t)(i - di) * n;
+        if (j - m >= 0 && skel[row + j - m]) return row + j - m;
+        if (m > 0 && j + m < n && skel[row + j + m]) return row + j + m;
     }
     return -1;
 }

@@ -186,8 +186,8 @@ def pore_properties_gpu(pore, dx, mfp, stream=None, return_iterations=False):
     n = pore.shape[0]
     if pore.shape != (n, n):
         raise ValueError("pore image must be square")
-    lp = np.zeros((n, n))
-    kn = np.zeros((n, n))
+    lp = np.empty((n, n))
+    kn = np.empty((n, n))
     it = C.c_int64(0)
     rc = lib().mgpu_pore_properties_gpu(pore.reshape(-1), n, dx, mfp, lp.reshape(-1), kn.reshape(-1),
                                         C.byref(it), stream)
