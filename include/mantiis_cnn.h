@@ -27,6 +27,12 @@ int cnn_conv3x3_forward(const float *x, const uint16_t *w, const float *b, float
 /* dx = the gradient of conv3x3 with respect to its input, from dy (cout channels) */
 int cnn_conv3x3_backward_data(const float *dy, const uint16_t *w, float *dx, int n, int cin, int cout, int h, int wd,
                               void *stream);
+/* The two calls above and the pass that follows each in the network, in one: sum = y + skip;
+ * masked = dx where the layer's input x > 0, else 0 (x the output of a ReLU).  y and dx may be NULL. */
+int cnn_conv3x3_forward_add(const float *x, const uint16_t *w, const float *b, float *y, const float *skip, float *sum,
+                            int n, int cin, int cout, int h, int wd, int relu, void *stream);
+int cnn_conv3x3_backward_data_relu(const float *dy, const uint16_t *w, float *dx, const float *x, float *masked, int n,
+                                   int cin, int cout, int h, int wd, void *stream);
 /* The same convolutions as implicit GEMMs on the tensor cores (tcgen05): the FP32
  * activations are split into two BF16 parts, each multiplied by the BF16 weights with FP32
  * accumulation in tensor memory, so the results agree with the two calls above to FP32
@@ -49,9 +55,14 @@ int cnn_relu_backward(float *dy, const float *y, int64_t count, void *stream);
 /* 2x2 mean pooling (h, wd even) and its adjoint */
 int cnn_avgpool2_forward(const float *x, float *y, int nc, int h, int wd, void *stream);
 int cnn_avgpool2_backward(const float *dy, float *dx, int nc, int h, int wd, void *stream);
+/* dx = dx + the adjoint where y > 0, else 0 */
+int cnn_avgpool2_backward_add_relu(const float *dy, const float *y, float *dx, int nc, int h, int wd, void *stream);
 /* nearest 2x upsampling of an (h, wd) map and its adjoint (sum of the 2x2 block) */
 int cnn_upsample2_forward(const float *x, float *y, int nc, int h, int wd, void *stream);
 int cnn_upsample2_backward(const float *dy, float *dx, int nc, int h, int wd, void *stream);
+/* the adjoint dx (may be NULL), and masked = dx where y > 0, else 0 */
+int cnn_upsample2_backward_relu(const float *dy, float *dx, const float *y, float *masked, int nc, int h, int wd,
+                                void *stream);
 /* y += x */
 int cnn_add(float *y, const float *x, int64_t count, void *stream);
 /* masked mean squared error over n images of c channels: loss[0] += sum mask (p - t)^2 / norm,
@@ -61,6 +72,17 @@ int cnn_mse(const float *p, const float *t, const float *mask, float *dp, float 
 /* Adam step on FP32 parameters, then their BF16 copy (w16 may be NULL) */
 int cnn_adam(float *w, const float *g, float *m, float *v, uint16_t *w16, int64_t count, float lr, float beta1,
              float beta2, float eps, int step, void *stream);
+/* The same for a list of parameter tensors (w16 may be NULL), and their gradients set to zero, in
+ * one launch per 32 tensors; the list itself is host memory, read before the call returns */
+typedef struct cnn_tensor
+{
+    float *w, *g, *m, *v;
+    uint16_t *w16;
+    int64_t count;
+} cnn_tensor;
+int cnn_adam_many(const cnn_tensor *tensors, int count, float lr, float beta1, float beta2, float eps, int step,
+                  void *stream);
+int cnn_zero_grad_many(const cnn_tensor *tensors, int count, void *stream);
 /* FP32 -> BF16 (round to nearest even) */
 int cnn_to_bf16(const float *x, uint16_t *y, int64_t count, void *stream);
 

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../../include/mantiis_cnn.h"
 #include "conv_fma.cuh"
@@ -21,53 +22,150 @@ __global__ void k_relu_bw(float *dy, const float *y, int64_t count)
     if (i < count && !(y[i] > 0.f)) dy[i] = 0.f;
 }
 
-// per (image * channel) plane: y (h/2, wd/2) = mean of the 2x2 blocks
-__global__ void k_pool_fw(const float *x, float *y, int nc, int h, int wd)
-{
-    const int ho = h / 2, wo = wd / 2;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)nc * ho * wo) return;
-    const int64_t c = i / ((int64_t)ho * wo);
-    const int r = (int)(i % ((int64_t)ho * wo)), yy = r / wo, xx = r % wo;
-    const float *p = x + c * h * wd + (int64_t)(2 * yy) * wd + 2 * xx;
-    y[i] = 0.25f * (p[0] + p[1] + p[wd] + p[wd + 1]);
-}
-
-__global__ void k_pool_bw(const float *dy, float *dx, int nc, int h, int wd)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)nc * h * wd) return;
-    const int64_t c = i / ((int64_t)h * wd);
-    const int r = (int)(i % ((int64_t)h * wd)), yy = r / wd, xx = r % wd;
-    dx[i] = 0.25f * dy[c * (h / 2) * (wd / 2) + (int64_t)(yy / 2) * (wd / 2) + xx / 2];
-}
-
-// nearest upsampling of an (h, wd) map to (2h, 2wd)
-__global__ void k_up_fw(const float *x, float *y, int nc, int h, int wd)
-{
-    const int ho = 2 * h, wo = 2 * wd;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)nc * ho * wo) return;
-    const int64_t c = i / ((int64_t)ho * wo);
-    const int r = (int)(i % ((int64_t)ho * wo)), yy = r / wo, xx = r % wo;
-    y[i] = x[c * h * wd + (int64_t)(yy / 2) * wd + xx / 2];
-}
-
-__global__ void k_up_bw(const float *dy, float *dx, int nc, int h, int wd)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)nc * h * wd) return;
-    const int64_t c = i / ((int64_t)h * wd);
-    const int r = (int)(i % ((int64_t)h * wd)), yy = r / wd, xx = r % wd;
-    const int wo = 2 * wd;
-    const float *p = dy + c * (4 * (int64_t)h * wd) + (int64_t)(2 * yy) * wo + 2 * xx;
-    dx[i] = p[0] + p[1] + p[wo] + p[wo + 1];
-}
-
 __global__ void k_add(float *y, const float *x, int64_t count)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count) y[i] += x[i];
+}
+
+// Pooling, upsampling and their adjoints.  What bounds them is memory (L2 for
+// most layers), as long as the index arithmetic is short: with 64-bit divisions
+// and one float per thread, upsampling 64 planes of 256^2 to 512^2 took 62 us, now
+// 13 (84 MB).  Each plane follows the last, so all are one image of coarse rows:
+// thread i takes V neighbouring pixels of a coarse row and the 2 x 2 V pixels of
+// the fine image that belong to them, as vectors (V = 2) where widths and
+// addresses allow; indices are 32-bit as long as they reach the end.  The passes
+// that followed one another over the same activations (the skip connection's sum,
+// ReLU adjoints, copies of a gradient for its two uses) are fused with these or
+// into the convolutions: of a training step on 8 x 128^2 they took 420 us, now 130.
+template <typename I, int V> struct Pixels
+{
+    I coarse, fine; // of the first pixel; the second fine row is 2 w further on
+    __device__ __forceinline__ Pixels(I i, int w)
+    {
+        const I per = (I)(w / V), r = i / per, c = (i - r * per) * V;
+        coarse = r * (I)w + c;
+        fine = r * 4 * (I)w + 2 * c;
+    }
+    static __device__ __forceinline__ void load(const float *p, float v[V])
+    {
+        if constexpr (V == 2)
+        {
+            const float2 q = *reinterpret_cast<const float2 *>(p);
+            v[0] = q.x, v[1] = q.y;
+        }
+        else v[0] = p[0];
+    }
+    static __device__ __forceinline__ void store(float *p, const float v[V])
+    {
+        if constexpr (V == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+        else p[0] = v[0];
+    }
+    static __device__ __forceinline__ void load_fine(const float *p, float v[2 * V])
+    {
+        if constexpr (V == 2)
+        {
+            const float4 q = *reinterpret_cast<const float4 *>(p);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        }
+        else v[0] = p[0], v[1] = p[1];
+    }
+    static __device__ __forceinline__ void store_fine(float *p, const float v[2 * V])
+    {
+        if constexpr (V == 2) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        else p[0] = v[0], p[1] = v[1];
+    }
+};
+
+// y (coarse) = mean of the 2x2 blocks of x
+template <typename I, int V> __global__ void k_pool_fw(const float *x, float *y, I count, int w)
+{
+    typedef Pixels<I, V> P;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const P p(i, w);
+    float a[2 * V], b[2 * V], m[V];
+    P::load_fine(x + p.fine, a);
+    P::load_fine(x + p.fine + 2 * w, b);
+#pragma unroll
+    for (int k = 0; k < V; k++) m[k] = 0.25f * (a[2 * k] + a[2 * k + 1] + b[2 * k] + b[2 * k + 1]);
+    P::store(y + p.coarse, m);
+}
+
+// its adjoint, dx (fine) = dy / 4
+template <typename I, int V> __global__ void k_pool_bw(const float *dy, float *dx, I count, int w)
+{
+    typedef Pixels<I, V> P;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const P p(i, w);
+    float g[V], f[2 * V];
+    P::load(dy + p.coarse, g);
+#pragma unroll
+    for (int k = 0; k < V; k++) f[2 * k] = f[2 * k + 1] = 0.25f * g[k];
+    P::store_fine(dx + p.fine, f);
+    P::store_fine(dx + p.fine + 2 * w, f);
+}
+
+// ... added to the gradient that the skip connection brought, and through the
+// ReLU that gave the fine y: dx = dx + dy / 4 where y > 0, else 0
+template <typename I, int V>
+__global__ void k_pool_bw_add_relu(const float *dy, const float *y, float *dx, I count, int w)
+{
+    typedef Pixels<I, V> P;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const P p(i, w);
+    float g[V];
+    P::load(dy + p.coarse, g);
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+    {
+        float v[2 * V], m[2 * V];
+        P::load_fine(y + p.fine + r * 2 * w, m);
+        P::load_fine(dx + p.fine + r * 2 * w, v);
+#pragma unroll
+        for (int k = 0; k < 2 * V; k++) v[k] = m[k] > 0.f ? v[k] + __fmul_rn(0.25f, g[k / 2]) : 0.f;
+        P::store_fine(dx + p.fine + r * 2 * w, v);
+    }
+}
+
+// y (fine) = nearest upsampling of x
+template <typename I, int V> __global__ void k_up_fw(const float *x, float *y, I count, int w)
+{
+    typedef Pixels<I, V> P;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const P p(i, w);
+    float v[V], f[2 * V];
+    P::load(x + p.coarse, v);
+#pragma unroll
+    for (int k = 0; k < V; k++) f[2 * k] = f[2 * k + 1] = v[k];
+    P::store_fine(y + p.fine, f);
+    P::store_fine(y + p.fine + 2 * w, f);
+}
+
+// its adjoint, dx (coarse, may be null) = sum of the 2x2 blocks of dy; with y, also
+// masked = dx through the ReLU that gave y
+template <typename I, int V>
+__global__ void k_up_bw(const float *dy, float *dx, const float *y, float *masked, I count, int w)
+{
+    typedef Pixels<I, V> P;
+    const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const P p(i, w);
+    float a[2 * V], b[2 * V], s[V];
+    P::load_fine(dy + p.fine, a);
+    P::load_fine(dy + p.fine + 2 * w, b);
+#pragma unroll
+    for (int k = 0; k < V; k++) s[k] = a[2 * k] + a[2 * k + 1] + b[2 * k] + b[2 * k + 1];
+    if (dx) P::store(dx + p.coarse, s);
+    if (!y) return;
+    float m[V];
+    P::load(y + p.coarse, m);
+#pragma unroll
+    for (int k = 0; k < V; k++) s[k] = m[k] > 0.f ? s[k] : 0.f;
+    P::store(masked + p.coarse, s);
 }
 
 __global__ void __launch_bounds__(256) k_mse(const float *p, const float *t, const float *mask, float *dp, float *loss,
@@ -95,19 +193,55 @@ __global__ void __launch_bounds__(256) k_mse(const float *p, const float *t, con
     if (threadIdx.x == 0) atomicAdd(loss, red[0]);
 }
 
-__global__ void k_adam(float *w, const float *g, float *m, float *v, uint16_t *w16, int64_t count, float lr, float b1,
-                       float b2, float eps, float c1, float c2)
+struct AdamRates
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ void adam_one(float *w, const float *g, float *m, float *v, uint16_t *w16, int64_t i,
+                                         const AdamRates &a)
+{
     const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+    const float mi = a.b1 * m[i] + (1.f - a.b1) * gi;
+    const float vi = a.b2 * v[i] + (1.f - a.b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float wi = w[i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
     w[i] = wi;
     if (w16) w16[i] = __bfloat16_as_ushort(__float2bfloat16_rn(wi));
+}
+
+// One launch for up to kListed tensors: block b belongs to the last tensor whose
+// first block is not after b.  The network's 22 tensors took 22 launches of 3 to
+// 6 us for the update and 22 of 2 us to clear the gradients; one of each: 19 and 10.
+constexpr int kListed = 32;
+struct TensorList
+{
+    cnn_tensor t[kListed];
+    unsigned first[kListed]; // block
+    int count;
+};
+__device__ __forceinline__ bool listed(const TensorList &list, int &k, int64_t &i)
+{
+    k = 0;
+    while (k + 1 < list.count && blockIdx.x >= list.first[k + 1]) k++;
+    i = (int64_t)(blockIdx.x - list.first[k]) * blockDim.x + threadIdx.x;
+    return i < list.t[k].count;
+}
+
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ TensorList list, AdamRates rates)
+{
+    int k;
+    int64_t i;
+    if (!listed(list, k, i)) return;
+    const cnn_tensor &t = list.t[k];
+    adam_one(t.w, t.g, t.m, t.v, t.w16, i, rates);
+}
+
+__global__ void __launch_bounds__(256) k_zero_grad(const __grid_constant__ TensorList list)
+{
+    int k;
+    int64_t i;
+    if (listed(list, k, i)) list.t[k].g[i] = 0.f;
 }
 
 __global__ void k_to_bf16(const float *x, uint16_t *y, int64_t count)
@@ -123,6 +257,50 @@ int done()
 }
 
 unsigned blocks(int64_t count) { return (unsigned)((count + 255) / 256); }
+
+// f(index type, pixels per thread, threads): two coarse pixels a thread where the
+// coarse width is even and all addresses (or'd together) are on 16 bytes
+template <typename F> int each_coarse(int64_t rows, int w, uintptr_t addresses, F f)
+{
+    const int64_t count = rows * w;
+    const bool narrow = 4 * count + 1024 < (int64_t)1 << 32;
+    if (w % 2 == 0 && addresses % 16 == 0)
+    {
+        if (narrow) f(uint32_t(), std::integral_constant<int, 2>(), count / 2);
+        else f(int64_t(), std::integral_constant<int, 2>(), count / 2);
+    }
+    else
+    {
+        if (narrow) f(uint32_t(), std::integral_constant<int, 1>(), count);
+        else f(int64_t(), std::integral_constant<int, 1>(), count);
+    }
+    return done();
+}
+inline uintptr_t address(const void *p) { return (uintptr_t)p; }
+
+// the list in launches of up to kListed tensors
+template <typename F> int each_listed(const cnn_tensor *tensors, int count, F launch)
+{
+    TensorList list;
+    int64_t total = 0;
+    list.count = 0;
+    for (int k = 0; k < count; k++)
+    {
+        const int64_t n = ((tensors[k].count > 0 ? tensors[k].count : 0) + 255) / 256;
+        if (list.count == kListed || total + n > INT32_MAX)
+        {
+            if (total) launch(list, (unsigned)total);
+            list.count = 0;
+            total = 0;
+        }
+        if (n == 0) continue;
+        list.t[list.count] = tensors[k];
+        list.first[list.count++] = (unsigned)total;
+        total += n;
+    }
+    if (total) launch(list, (unsigned)total);
+    return done();
+}
 
 // the tensor-core convolutions take more than 48 KB of dynamic shared memory
 int tc_attributes()
@@ -182,8 +360,8 @@ cudaError_t allow_smem(const void *kernel, size_t bytes, std::atomic<uint64_t> &
 }
 
 template <typename T, bool TRANSPOSE>
-int launch_conv(const float *x, const uint16_t *w, const float *b, float *y, int n, int cin, int cout, int h, int wd,
-                int relu, cudaStream_t st)
+int launch_conv(const float *x, const uint16_t *w, const float *b, float *y, const float *extra, float *y2, int n, int cin,
+                int cout, int h, int wd, int relu, cudaStream_t st)
 {
     static std::atomic<uint64_t> ready{0};
     const auto kernel = cnn_fma::k_conv3x3_fma<T, TRANSPOSE>;
@@ -191,7 +369,7 @@ int launch_conv(const float *x, const uint16_t *w, const float *b, float *y, int
     if (e != cudaSuccess) return -(int)e;
     const dim3 grid((unsigned)(((wd + T::TW - 1) / T::TW) * ((h + T::TH - 1) / T::TH)),
                     (unsigned)((cout + T::CO - 1) / T::CO), (unsigned)n);
-    kernel<<<grid, T::kThreads, T::kSmem, st>>>(x, w, b, y, cin, cout, h, wd, relu);
+    kernel<<<grid, T::kThreads, T::kSmem, st>>>(x, w, b, y, extra, y2, cin, cout, h, wd, relu);
     return done();
 }
 
@@ -216,8 +394,8 @@ template <typename T> double conv_cost(int n, int cout, int h, int wd, int sms, 
 }
 
 template <bool TRANSPOSE>
-int conv(const float *x, const uint16_t *w, const float *b, float *y, int n, int cin, int cout, int h, int wd, int relu,
-         cudaStream_t st)
+int conv(const float *x, const uint16_t *w, const float *b, float *y, const float *extra, float *y2, int n, int cin,
+         int cout, int h, int wd, int relu, cudaStream_t st)
 {
     const int sms = sm_count();
     const double cost[5] = {conv_cost<ConvA>(n, cout, h, wd, sms, 1.0), conv_cost<ConvB>(n, cout, h, wd, sms, 1.06),
@@ -225,11 +403,11 @@ int conv(const float *x, const uint16_t *w, const float *b, float *y, int n, int
                             conv_cost<ConvE>(n, cout, h, wd, sms, 1.5)};
     switch ((int)(std::min_element(cost, cost + 5) - cost))
     {
-    case 0: return launch_conv<ConvA, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
-    case 1: return launch_conv<ConvB, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
-    case 2: return launch_conv<ConvC, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
-    case 3: return launch_conv<ConvD, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
-    default: return launch_conv<ConvE, TRANSPOSE>(x, w, b, y, n, cin, cout, h, wd, relu, st);
+    case 0: return launch_conv<ConvA, TRANSPOSE>(x, w, b, y, extra, y2, n, cin, cout, h, wd, relu, st);
+    case 1: return launch_conv<ConvB, TRANSPOSE>(x, w, b, y, extra, y2, n, cin, cout, h, wd, relu, st);
+    case 2: return launch_conv<ConvC, TRANSPOSE>(x, w, b, y, extra, y2, n, cin, cout, h, wd, relu, st);
+    case 3: return launch_conv<ConvD, TRANSPOSE>(x, w, b, y, extra, y2, n, cin, cout, h, wd, relu, st);
+    default: return launch_conv<ConvE, TRANSPOSE>(x, w, b, y, extra, y2, n, cin, cout, h, wd, relu, st);
     }
 }
 
@@ -256,7 +434,14 @@ int cnn_conv3x3_forward(const float *x, const uint16_t *w, const float *b, float
                         int wd, int relu, void *stream)
 {
     if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0) return -1;
-    return conv<false>(x, w, b, y, n, cin, cout, h, wd, relu, (cudaStream_t)stream);
+    return conv<false>(x, w, b, y, nullptr, nullptr, n, cin, cout, h, wd, relu, (cudaStream_t)stream);
+}
+
+int cnn_conv3x3_forward_add(const float *x, const uint16_t *w, const float *b, float *y, const float *skip, float *sum,
+                            int n, int cin, int cout, int h, int wd, int relu, void *stream)
+{
+    if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0 || !skip || !sum) return -1;
+    return conv<false>(x, w, b, y, skip, sum, n, cin, cout, h, wd, relu, (cudaStream_t)stream);
 }
 
 int cnn_conv3x3_backward_data(const float *dy, const uint16_t *w, float *dx, int n, int cin, int cout, int h, int wd,
@@ -264,7 +449,14 @@ int cnn_conv3x3_backward_data(const float *dy, const uint16_t *w, float *dx, int
 {
     if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0) return -1;
     // a convolution from the cout gradient channels to the cin input channels
-    return conv<true>(dy, w, nullptr, dx, n, cout, cin, h, wd, 0, (cudaStream_t)stream);
+    return conv<true>(dy, w, nullptr, dx, nullptr, nullptr, n, cout, cin, h, wd, 0, (cudaStream_t)stream);
+}
+
+int cnn_conv3x3_backward_data_relu(const float *dy, const uint16_t *w, float *dx, const float *x, float *masked, int n,
+                                   int cin, int cout, int h, int wd, void *stream)
+{
+    if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0 || !x || !masked) return -1;
+    return conv<true>(dy, w, nullptr, dx, x, masked, n, cout, cin, h, wd, 0, (cudaStream_t)stream);
 }
 
 int cnn_conv3x3_forward_tc(const float *x, const uint16_t *w, const float *b, float *y, int n, int cin, int cout,
@@ -354,29 +546,59 @@ int cnn_relu_backward(float *dy, const float *y, int64_t count, void *stream)
 int cnn_avgpool2_forward(const float *x, float *y, int nc, int h, int wd, void *stream)
 {
     if (nc <= 0 || h <= 0 || wd <= 0 || h % 2 || wd % 2) return -1;
-    k_pool_fw<<<blocks((int64_t)nc * h * wd / 4), 256, 0, (cudaStream_t)stream>>>(x, y, nc, h, wd);
-    return done();
+    return each_coarse((int64_t)nc * (h / 2), wd / 2, address(x) | address(y), [&](auto i, auto v, int64_t count) {
+        typedef decltype(i) I;
+        k_pool_fw<I, v><<<blocks(count), 256, 0, (cudaStream_t)stream>>>(x, y, (I)count, wd / 2);
+    });
 }
 
 int cnn_avgpool2_backward(const float *dy, float *dx, int nc, int h, int wd, void *stream)
 {
     if (nc <= 0 || h <= 0 || wd <= 0 || h % 2 || wd % 2) return -1;
-    k_pool_bw<<<blocks((int64_t)nc * h * wd), 256, 0, (cudaStream_t)stream>>>(dy, dx, nc, h, wd);
-    return done();
+    return each_coarse((int64_t)nc * (h / 2), wd / 2, address(dy) | address(dx), [&](auto i, auto v, int64_t count) {
+        typedef decltype(i) I;
+        k_pool_bw<I, v><<<blocks(count), 256, 0, (cudaStream_t)stream>>>(dy, dx, (I)count, wd / 2);
+    });
+}
+
+int cnn_avgpool2_backward_add_relu(const float *dy, const float *y, float *dx, int nc, int h, int wd, void *stream)
+{
+    if (nc <= 0 || h <= 0 || wd <= 0 || h % 2 || wd % 2) return -1;
+    return each_coarse((int64_t)nc * (h / 2), wd / 2, address(dy) | address(y) | address(dx),
+                       [&](auto i, auto v, int64_t count) {
+                           typedef decltype(i) I;
+                           k_pool_bw_add_relu<I, v><<<blocks(count), 256, 0, (cudaStream_t)stream>>>(dy, y, dx, (I)count, wd / 2);
+                       });
 }
 
 int cnn_upsample2_forward(const float *x, float *y, int nc, int h, int wd, void *stream)
 {
     if (nc <= 0 || h <= 0 || wd <= 0) return -1;
-    k_up_fw<<<blocks((int64_t)nc * h * wd * 4), 256, 0, (cudaStream_t)stream>>>(x, y, nc, h, wd);
-    return done();
+    return each_coarse((int64_t)nc * h, wd, address(x) | address(y), [&](auto i, auto v, int64_t count) {
+        typedef decltype(i) I;
+        k_up_fw<I, v><<<blocks(count), 256, 0, (cudaStream_t)stream>>>(x, y, (I)count, wd);
+    });
+}
+
+static int upsample2_backward(const float *dy, float *dx, const float *y, float *masked, int nc, int h, int wd, void *stream)
+{
+    if (nc <= 0 || h <= 0 || wd <= 0) return -1;
+    return each_coarse((int64_t)nc * h, wd, address(dy) | address(dx) | address(y) | address(masked),
+                       [&](auto i, auto v, int64_t count) {
+                           typedef decltype(i) I;
+                           k_up_bw<I, v><<<blocks(count), 256, 0, (cudaStream_t)stream>>>(dy, dx, y, masked, (I)count, wd);
+                       });
 }
 
 int cnn_upsample2_backward(const float *dy, float *dx, int nc, int h, int wd, void *stream)
 {
-    if (nc <= 0 || h <= 0 || wd <= 0) return -1;
-    k_up_bw<<<blocks((int64_t)nc * h * wd), 256, 0, (cudaStream_t)stream>>>(dy, dx, nc, h, wd);
-    return done();
+    return upsample2_backward(dy, dx, nullptr, nullptr, nc, h, wd, stream);
+}
+
+int cnn_upsample2_backward_relu(const float *dy, float *dx, const float *y, float *masked, int nc, int h, int wd, void *stream)
+{
+    if (!y || !masked) return -1;
+    return upsample2_backward(dy, dx, y, masked, nc, h, wd, stream);
 }
 
 int cnn_add(float *y, const float *x, int64_t count, void *stream)
@@ -394,14 +616,28 @@ int cnn_mse(const float *p, const float *t, const float *mask, float *dp, float 
     return done();
 }
 
+int cnn_adam_many(const cnn_tensor *tensors, int count, float lr, float beta1, float beta2, float eps, int step, void *stream)
+{
+    if (step < 1) return -1;
+    const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
+    return each_listed(tensors, count, [&](const TensorList &list, unsigned blocks) {
+        k_adam<<<blocks, 256, 0, (cudaStream_t)stream>>>(list, AdamRates{lr, beta1, beta2, eps, c1, c2});
+    });
+}
+
 int cnn_adam(float *w, const float *g, float *m, float *v, uint16_t *w16, int64_t count, float lr, float beta1,
              float beta2, float eps, int step, void *stream)
 {
     if (count <= 0) return 0;
-    if (step < 1) return -1;
-    const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-    k_adam<<<blocks(count), 256, 0, (cudaStream_t)stream>>>(w, g, m, v, w16, count, lr, beta1, beta2, eps, c1, c2);
-    return done();
+    const cnn_tensor t{w, const_cast<float *>(g), m, v, w16, count};
+    return cnn_adam_many(&t, 1, lr, beta1, beta2, eps, step, stream);
+}
+
+int cnn_zero_grad_many(const cnn_tensor *tensors, int count, void *stream)
+{
+    return each_listed(tensors, count, [&](const TensorList &list, unsigned blocks) {
+        k_zero_grad<<<blocks, 256, 0, (cudaStream_t)stream>>>(list);
+    });
 }
 
 int cnn_to_bf16(const float *x, uint16_t *y, int64_t count, void *stream)

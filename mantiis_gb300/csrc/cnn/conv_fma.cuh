@@ -80,11 +80,15 @@ template <int TW_, int TH_, int PY_, int CG_, int CT_, int CI_> struct ConvTile
 // with k = 3 ky + kx, zero outside the image; summed with ci ascending, then k
 // ascending, whatever the tile.  TRANSPOSE: the data gradient of such a
 // convolution, i.e. the same with w[ci][co][8 - k]; cin and cout are this
-// convolution's own input / output channel counts.
+// convolution's own input / output channel counts.  With y2 (y may then be null)
+// the pass over the result that follows in the network is done on the way out:
+// y2 = y + extra (the decoder's skip connection) or, TRANSPOSE, y2 = y where
+// extra > 0, else 0 (the adjoint of the ReLU that gave extra).
 template <typename T, bool TRANSPOSE>
 __global__ void __launch_bounds__(T::kThreads, 512 / T::kThreads)
     k_conv3x3_fma(const float *__restrict__ x, const uint16_t *__restrict__ w, const float *__restrict__ b,
-                  float *__restrict__ y, int cin, int cout, int h, int wd, int relu)
+                  float *__restrict__ y, const float *__restrict__ extra, float *__restrict__ y2, int cin, int cout,
+                  int h, int wd, int relu)
 {
     extern __shared__ __align__(16) float smem[];
     const int tid = (int)threadIdx.x;
@@ -275,7 +279,16 @@ __global__ void __launch_bounds__(T::kThreads, 512 / T::kThreads)
     const int gx = tx0 + px;
     if (gx >= wd) return;
     // whole groups of 4 pixels are one store where rows start on 16 bytes
-    const bool vec = (wd & 3) == 0 && ((uintptr_t)y & 15u) == 0;
+    const bool vec = (wd & 3) == 0 && (((uintptr_t)y | (uintptr_t)extra | (uintptr_t)y2) & 15u) == 0;
+    auto put = [&](float *dst, const float v[kPX]) {
+        if (vec) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        else
+        {
+#pragma unroll
+            for (int p = 0; p < kPX; p++)
+                if (gx + p < wd) dst[p] = v[p];
+        }
+    };
 #pragma unroll
     for (int o = 0; o < T::CT; o++)
     {
@@ -294,14 +307,23 @@ __global__ void __launch_bounds__(T::kThreads, 512 / T::kThreads)
                 v[p] = half_of(acc[a][p][o / 2], o & 1) + bias;
                 if (relu) v[p] = fmaxf(v[p], 0.f);
             }
-            float *dst = y + ((size_t)img * cout + gco) * plane + (size_t)gy * wd + gx;
-            if (vec) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            const size_t at = ((size_t)img * cout + gco) * plane + (size_t)gy * wd + gx;
+            if (y) put(y + at, v);
+            if (!y2) continue;
+            float e[kPX];
+            if (vec)
+            {
+                const float4 q = *reinterpret_cast<const float4 *>(extra + at);
+                e[0] = q.x, e[1] = q.y, e[2] = q.z, e[3] = q.w;
+            }
             else
             {
 #pragma unroll
-                for (int p = 0; p < kPX; p++)
-                    if (gx + p < wd) dst[p] = v[p];
+                for (int p = 0; p < kPX; p++) e[p] = gx + p < wd ? extra[at + p] : 0.f;
             }
+#pragma unroll
+            for (int p = 0; p < kPX; p++) v[p] = TRANSPOSE ? (e[p] > 0.f ? v[p] : 0.f) : v[p] + e[p];
+            put(y2 + at, v);
         }
     }
 }

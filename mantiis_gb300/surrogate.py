@@ -42,6 +42,8 @@ _P = C.c_void_p
 _SIG = {
     "cnn_conv3x3_forward": [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P],
     "cnn_conv3x3_backward_data": [_P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P],
+    "cnn_conv3x3_forward_add": [_P, _P, _P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P],
+    "cnn_conv3x3_backward_data_relu": [_P, _P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P],
     "cnn_conv3x3_forward_tc": [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P],
     "cnn_conv3x3_backward_data_tc": [_P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P],
     "cnn_conv3x3_backward_weight_tc": [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _P],
@@ -50,13 +52,22 @@ _SIG = {
     "cnn_relu_backward": [_P, _P, C.c_int64, _P],
     "cnn_avgpool2_forward": [_P, _P, C.c_int, C.c_int, C.c_int, _P],
     "cnn_avgpool2_backward": [_P, _P, C.c_int, C.c_int, C.c_int, _P],
+    "cnn_avgpool2_backward_add_relu": [_P, _P, _P, C.c_int, C.c_int, C.c_int, _P],
     "cnn_upsample2_forward": [_P, _P, C.c_int, C.c_int, C.c_int, _P],
     "cnn_upsample2_backward": [_P, _P, C.c_int, C.c_int, C.c_int, _P],
+    "cnn_upsample2_backward_relu": [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, _P],
     "cnn_add": [_P, _P, C.c_int64, _P],
     "cnn_mse": [_P, _P, _P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_float, _P],
     "cnn_adam": [_P, _P, _P, _P, _P, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int, _P],
+    "cnn_adam_many": [_P, C.c_int, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int, _P],
+    "cnn_zero_grad_many": [_P, C.c_int, _P],
     "cnn_to_bf16": [_P, _P, C.c_int64, _P],
 }
+
+
+class _Tensor(C.Structure):
+    """cnn_tensor: a parameter, its gradient, moments and BF16 copy."""
+    _fields_ = [("w", _P), ("g", _P), ("m", _P), ("v", _P), ("w16", _P), ("count", C.c_int64)]
 
 
 def cnn_lib():
@@ -117,18 +128,33 @@ class Conv3x3:
     def sync_bf16(self):
         _check(cnn_lib().cnn_to_bf16(_ptr(self.w), _ptr(self.w16), self.w.numel(), _stream()), "to_bf16")
 
-    def forward(self, x, relu):
+    def forward(self, x, relu, skip=None, keep=True):
+        """The layer's output y; with skip, (y, y + skip), where y is None without keep."""
         import torch
 
         n, _, h, w = x.shape
-        y = torch.empty((n, self.cout, h, w), dtype=torch.float32, device="cuda")
+        shape = (n, self.cout, h, w)
+        if skip is not None and tuple(skip.shape) != shape:
+            raise ValueError(f"skip connection of shape {tuple(skip.shape)}, output {shape}")
+        new = lambda: torch.empty(shape, dtype=torch.float32, device="cuda")
+        if skip is not None and not TENSOR_CORES:
+            y, d = new() if keep else None, new()
+            _check(cnn_lib().cnn_conv3x3_forward_add(_ptr(x), _ptr(self.w16), _ptr(self.b), _ptr(y), _ptr(skip),
+                                                     _ptr(d), n, self.cin, self.cout, h, w, 1 if relu else 0,
+                                                     _stream()), "conv forward")
+            return y, d
+        y = new()
         fwd = cnn_lib().cnn_conv3x3_forward_tc if TENSOR_CORES else cnn_lib().cnn_conv3x3_forward
         _check(fwd(_ptr(x), _ptr(self.w16), _ptr(self.b), _ptr(y), n, self.cin, self.cout, h, w, 1 if relu else 0,
                    _stream()), "conv forward")
-        return y
+        if skip is None:
+            return y
+        return (y, _add(y.clone(), skip)) if keep else (None, _add(y, skip))
 
-    def backward(self, x, dy, need_dx=True):
-        """Accumulates dw, db from the layer input x and output gradient dy; returns dx."""
+    def backward(self, x, dy, need_dx=True, relu=None, keep=True):
+        """Accumulates dw, db from the layer input x and output gradient dy; returns dx.
+        With relu, an output of that shape of a ReLU, (dx, dx through that ReLU), where dx
+        is None without keep."""
         import torch
 
         n, _, h, w = x.shape
@@ -137,10 +163,25 @@ class Conv3x3:
                                              h, w, _stream()), "conv weight gradient")
         if not need_dx:
             return None
+        if relu is not None and relu.shape != x.shape:
+            raise ValueError(f"ReLU output of shape {tuple(relu.shape)}, layer input {tuple(x.shape)}")
+        if relu is not None and not TENSOR_CORES:
+            dx, masked = torch.empty_like(x) if keep else None, torch.empty_like(x)
+            _check(L.cnn_conv3x3_backward_data_relu(_ptr(dy), _ptr(self.w16), _ptr(dx), _ptr(relu), _ptr(masked), n,
+                                                    self.cin, self.cout, h, w, _stream()), "conv data gradient")
+            return dx, masked
         dx = torch.empty_like(x)
         bwd = L.cnn_conv3x3_backward_data_tc if TENSOR_CORES else L.cnn_conv3x3_backward_data
         _check(bwd(_ptr(dy), _ptr(self.w16), _ptr(dx), n, self.cin, self.cout, h, w, _stream()), "conv data gradient")
-        return dx
+        if relu is None:
+            return dx
+        return (dx, _relu_bw(dx.clone(), relu)) if keep else (None, _relu_bw(dx, relu))
+
+    def tensors(self):
+        """The layer's two cnn_tensor entries."""
+        w, b = self.state[:2], self.state[2:]
+        return [(_ptr(self.w), _ptr(self.dw), _ptr(w[0]), _ptr(w[1]), _ptr(self.w16), self.w.numel()),
+                (_ptr(self.b), _ptr(self.db), _ptr(b[0]), _ptr(b[1]), None, self.b.numel())]
 
     def zero_grad(self):
         self.dw.zero_()
@@ -168,12 +209,10 @@ def _pool(x):
     return y
 
 
-def _pool_bw(dy, shape):
-    import torch
-
-    n, c, h, w = shape
-    dx = torch.empty(shape, dtype=torch.float32, device="cuda")
-    _check(cnn_lib().cnn_avgpool2_backward(_ptr(dy), _ptr(dx), n * c, h, w, _stream()), "pool backward")
+def _pool_bw_add_relu(dx, dy, y):
+    n, c, h, w = dx.shape
+    _check(cnn_lib().cnn_avgpool2_backward_add_relu(_ptr(dy), _ptr(y), _ptr(dx), n * c, h, w, _stream()),
+           "pool backward")
     return dx
 
 
@@ -186,14 +225,14 @@ def _up(x):
     return y
 
 
-def _up_bw(dy):
+def _up_bw_relu(dy, y, keep=True):
     import torch
 
-    n, c, h2, w2 = dy.shape
-    dx = torch.empty((n, c, h2 // 2, w2 // 2), dtype=torch.float32, device="cuda")
-    _check(cnn_lib().cnn_upsample2_backward(_ptr(dy), _ptr(dx), n * c, h2 // 2, w2 // 2, _stream()),
+    n, c, h, w = y.shape
+    dx, masked = torch.empty_like(y) if keep else None, torch.empty_like(y)
+    _check(cnn_lib().cnn_upsample2_backward_relu(_ptr(dy), _ptr(dx), _ptr(y), _ptr(masked), n * c, h, w, _stream()),
            "upsample backward")
-    return dx
+    return dx, masked
 
 
 def _add(y, x):
@@ -233,8 +272,7 @@ class UNet:
         u, c = {}, {}
         for k, i in enumerate(range(3, -1, -1)):
             u[i] = _up(d[i + 1])
-            c[i] = self.dec[k].forward(u[i], True)
-            d[i] = _add(c[i].clone(), e[i])
+            c[i], d[i] = self.dec[k].forward(u[i], True, skip=e[i], keep=keep)
         y = self.out.forward(d[0], False)
         if keep:
             a.update(e=e, p=p, u=u, c=c, d=d)
@@ -244,32 +282,29 @@ class UNet:
     def backward(self, dy):
         a = self._acts
         e, p, u, c, d = a["e"], a["p"], a["u"], a["c"], a["d"]
-        dd = self.out.backward(d[0], dy)
+        # d[i] = c[i] + e[i]: the gradient reaches the skip (de) and, through its
+        # ReLU, the decoder's convolution (g); d[4] = e[4]
         de = {}
+        de[0], g = self.out.backward(d[0], dy, relu=c[0])
         for i in range(0, 4):
-            # d[i] = c[i] + e[i]: the gradient reaches the skip and the decoder conv
-            de[i] = dd.clone()
-            dc = _relu_bw(dd, c[i])
-            du = self.dec[3 - i].backward(u[i], dc)
-            dd = _up_bw(du)  # gradient of d[i + 1]
-        de[4] = dd
+            du = self.dec[3 - i].backward(u[i], g)
+            de[i + 1], g = _up_bw_relu(du, c[i + 1] if i < 3 else e[4], keep=i < 3)
         for i in range(4, 0, -1):
-            g = _relu_bw(de[i], e[i])
             dp = self.enc[i - 1].backward(p[i], g)
-            _add(de[i - 1], _pool_bw(dp, tuple(e[i - 1].shape)))
-        g = _relu_bw(de[0], e[0])
-        da0 = self.enc0b.backward(a["a0"], g)
-        g = _relu_bw(da0, a["a0"])
+            g = _pool_bw_add_relu(de[i - 1], dp, e[i - 1])
+        _, g = self.enc0b.backward(a["a0"], g, relu=a["a0"], keep=False)
         self.enc0a.backward(a["x"], g, need_dx=False)
 
+    def _tensors(self):
+        t = [e for l in self.layers() for e in l.tensors()]
+        return (_Tensor * len(t))(*t), len(t)
+
     def zero_grad(self):
-        for l in self.layers():
-            l.zero_grad()
+        _check(cnn_lib().cnn_zero_grad_many(*self._tensors(), _stream()), "zero_grad")
 
     def adam(self, lr):
         self.step += 1
-        for l in self.layers():
-            l.adam(lr, self.step)
+        _check(cnn_lib().cnn_adam_many(*self._tensors(), lr, 0.9, 0.999, 1e-8, self.step, _stream()), "adam")
 
 
 def masked_loss(pred, target, mask):
