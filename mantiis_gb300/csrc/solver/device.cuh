@@ -22,9 +22,10 @@ namespace dev
 {
 // boundary tables in constant memory: specular target per (type, direction),
 // and per type the directions with c.n > 0 and c.n < 0 (MDBB)
-// specular targets per boundary type, in global memory: lanes of a warp index it
-// with different types, which the constant cache would serialize
-__device__ unsigned char c_icsr[MANTIIS_N_BND_TYPES * 9];
+// specular targets per boundary type, four bits for each link q, in global memory:
+// lanes of a warp index it with different types, which the constant cache would
+// serialize
+__device__ unsigned long long c_targets[MANTIIS_N_BND_TYPES];
 __constant__ unsigned short c_npos[MANTIIS_N_BND_TYPES];
 __constant__ unsigned short c_nneg[MANTIIS_N_BND_TYPES];
 struct LevelView
@@ -350,68 +351,78 @@ __device__ __forceinline__ void store_post(const LevelView &L, int x, int y, con
     }
 }
 
-// value of wall link q of cell (x, y) left by the previous step (parity 1-P)
-template <int P> __device__ __forceinline__ float wall_slot(const LevelView &L, int x, int y, int q)
+// where the previous step (parity 1-P) left the value of wall link q of cell (x, y)
+template <int P> __device__ __forceinline__ const float *wall_slot(const LevelView &L, int x, int y, int q)
 {
-    if (P == 1) return L.f[d2q9::opp(q) * L.plane + site_of(L, x, y)];
+    if (P == 1) return &L.f[d2q9::opp(q) * L.plane + site_of(L, x, y)];
     const int xd = wrapx(x + d2q9::cx(q), L.W), yd = wrapx(y + d2q9::cy(q), L.H);
-    return L.f[q * L.plane + site_of(L, xd, yd)];
+    return &L.f[q * L.plane + site_of(L, xd, yd)];
 }
 
 // Populations of a special cell after streaming and the wall rules:
 //   stream (=) -> wall (SRBB +=, BB/MDBB =) -> x-periodic (=) -> inlet/outlet (=)
 // (include/mantiisApp.hpp:239-265, include/coreLB.hpp:834-1009).  `raw` holds
-// the slots the cell reads at parity P; `wall(q)` gives the value its wall
-// link q left in the previous step.
+// the slots the cell reads at parity P; `wall_at(q)` gives where its wall link q
+// (1 to 8) left its value in the previous step.
+//
+// A warp of such cells is what the small images wait for in every step, and it is
+// bound by its instructions, one after the other: 4400 of a step's 9900 cycles on
+// 128^2 when each link was a branch with its own table load and quirk lookup.  The
+// links' work is therefore predicated, without branches, the specular targets are
+// one word, and the rare quirk values are read apart: a step 4.8 -> 3.7 us.
 template <typename WallSlot>
 __device__ __forceinline__ void special_rules(const Common &C, const SpecialRec &rec, int parity, int wall_mode,
-                                              const float raw[9], WallSlot wall_of, float df[9])
+                                              const float raw[9], WallSlot wall_at, float df[9])
 {
     const uint32_t arrive = rec.m0 & 0x1FFu, over = (rec.m0 >> 9) & 0x1FFu, wall = (rec.m0 >> 18) & 0x1FFu;
     const uint32_t quirk = rec.m1 & 0x1FFu, bnd = (rec.m1 >> 9) & 0xFFu, flags = (rec.m1 >> 17) & 0xFu;
-    // every load first (wall values, quirk values, constant terms, specular
-    // targets), so they are in flight together; then the arithmetic in the
-    // reference's order
-    const float *side_prev = C.side + (size_t)(parity ^ 1) * C.n_quirk;
+    // every load first (wall values, constant terms, specular targets), so they
+    // are in flight together; then the arithmetic in the reference's order
     float v[9], kq[9];
-    int p2s[9];
+    v[0] = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 9; q++)
+    for (int q = 1; q < 9; q++)
     {
+        const float *at = wall_at(q);
         v[q] = 0.0f;
-        p2s[q] = d2q9::opp(q);
-        if ((wall >> q) & 1u)
-        {
-            v[q] = ((quirk >> q) & 1u) ? side_prev[rec.quirk_base + __popc(quirk & ((1u << q) - 1u))] : wall_of(q);
-            if (bnd != 0xFFu) p2s[q] = (int)__ldg(&c_icsr[bnd * 9 + q]);
-        }
+        if ((wall >> q) & 1u) v[q] = *at;
     }
+    unsigned long long targets = 0x658721430ull; // the opposite directions
+    if (wall_mode == WALL_SRBB && bnd != 0xFFu) targets = __ldg(&c_targets[bnd]);
     const bool has_k = (flags & SF_HAS_K) != 0;
     const float *k = C.ktab + (size_t)(has_k ? rec.k_row : 0) * 9;
 #pragma unroll
     for (int q = 0; q < 9; q++) kq[q] = has_k ? __ldg(&k[q]) : 0.0f;
+    if (quirk & wall)
+    {
+        const float *side_prev = C.side + (size_t)(parity ^ 1) * C.n_quirk + rec.quirk_base;
+#pragma unroll
+        for (int q = 1; q < 9; q++)
+            if ((quirk & wall) >> q & 1u) v[q] = side_prev[__popc(quirk & ((1u << q) - 1u))];
+    }
 #pragma unroll
     for (int q = 0; q < 9; q++) df[q] = ((arrive >> q) & 1u) ? raw[q] : 0.0f;
     if (wall)
     {
-        const float r = rec.r;
+        const float r = rec.r, rs = 1.0f - r;
         // unrolled with fixed indices (the specular target is matched against
         // each population), so df stays in registers
 #pragma unroll
-        for (int q = 0; q < 9; q++)
+        for (int q = 1; q < 9; q++)
         {
-            if (!((wall >> q) & 1u)) continue;
+            const bool on = (wall >> q) & 1u;
             const int p1 = d2q9::opp(q);
             if (wall_mode == WALL_SRBB)
             {
-                const int p2 = p2s[q];
-                if (!((over >> p1) & 1u)) df[p1] += r * v[q];
-                const float rv = (((over >> p2) & 1u) ? 0.0f : (1.0f - r) * v[q]);
+                const uint32_t p2 = (uint32_t)(targets >> (4 * q)) & 15u;
+                if (on && !((over >> p1) & 1u)) df[p1] = __fmaf_rn(r, v[q], df[p1]);
+                const float rv = ((over >> p2) & 1u) ? 0.0f : __fmul_rn(rs, v[q]);
+                const uint32_t to = on ? p2 : 0u; // 0 is no link's target
 #pragma unroll
-                for (int p = 0; p < 9; p++)
-                    if (p == p2) df[p] += rv;
+                for (int p = 1; p < 9; p++)
+                    if (to == (uint32_t)p) df[p] = __fadd_rn(df[p], rv);
             }
-            else if (!((over >> p1) & 1u))
+            else if (on && !((over >> p1) & 1u))
                 df[p1] = v[q];
         }
     }

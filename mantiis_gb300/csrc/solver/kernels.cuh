@@ -1681,10 +1681,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_ads_persistent(const __grid_cons
 // memory.  A cell's populations are then the only round trip to memory.
 //
 // Measured on a GB300, us per coarse step without / with residuals: single block
-// 64^2 4.4 / 5.5, 128^2 4.8 / 5.9, 512^2 6.3 / 7.6, 1024^2 12.3 / 16.2, two levels
-// 256^2 18.6 / 20.0, 1024^2 34 / 37; the launches per phase 6.1 / 10.7, 6.2 / 10.4,
+// 64^2 3.6 / 4.4, 128^2 3.7 / 4.5, 512^2 5.3 / 7.1, 1024^2 12.1 / 15.5, two levels
+// 256^2 16.1 / 17.6, 1024^2 34 / 37; the launches per phase 6.1 / 10.7, 6.2 / 10.4,
 // 9.3 / 17.4, 16.4 / 34.7, 22.9 / 27.5, 42.8 / 55.9.  A grid barrier takes 0.85 us,
-// a warp of special cells about 3.5: what small images wait for.  At 1024^2 the
+// a warp of special cells about 2.5: what small images wait for.  At 1024^2 the
 // stages move 1.7 (single block) to 4 times (two levels: thin bands of fine cells)
 // the cells' bytes, whole sectors, between L2 and the SMs.
 constexpr int kMaxCoopDescs = 40, kMaxCoopPairs = 30;
@@ -1903,7 +1903,7 @@ __device__ __forceinline__ void coop_special(const CoopDesc &D, const CoopStep &
             // a wall link's value lies where the previous step stored it
             const CoopSlots before(L, stride, site, par ^ 1);
             special_rules(D.C, rec, par, st.wall, raw,
-                          [&](int q) { return L.f[par ? before.at[d2q9::opp(q)] : before.at[q]]; }, df);
+                          [&](int q) { return &L.f[par ? before.at[d2q9::opp(q)] : before.at[q]]; }, df);
         }
     }
     coop_collide<HEAVY, RES>(D, st, s, df, L.snap ? L.snap + s : nullptr, L.plane, sn, rec.omega, rec, unorm, acc, fs);

@@ -486,20 +486,22 @@ void encode_level_map(CUtensorMap *map, float *f, const LevelLayout &ll)
 
 void upload_constants()
 {
-    unsigned char icsr[MANTIIS_N_BND_TYPES * 9];
+    unsigned long long targets[MANTIIS_N_BND_TYPES];
     unsigned short npos[MANTIIS_N_BND_TYPES], nneg[MANTIIS_N_BND_TYPES];
     for (int t = 0; t < MANTIIS_N_BND_TYPES; t++)
     {
         npos[t] = nneg[t] = 0;
+        targets[t] = 0;
         for (int q = 0; q < 9; q++)
         {
-            icsr[t * 9 + q] = MANTIIS_ICSR[t][q];
+            targets[t] |= (unsigned long long)MANTIIS_ICSR[t][q] << (4 * q);
+            if (q && !MANTIIS_ICSR[t][q]) throw std::logic_error("a wall link reflects into the rest population");
             double cn = d2q9::CY[q] * MANTIIS_XY_NORM[t][1] + d2q9::CX[q] * MANTIIS_XY_NORM[t][0];
             if (cn > 0) npos[t] |= (unsigned short)(1u << q);
             else if (cn < 0) nneg[t] |= (unsigned short)(1u << q);
         }
     }
-    CK(cudaMemcpyToSymbol(dev::c_icsr, icsr, sizeof(icsr)));
+    CK(cudaMemcpyToSymbol(dev::c_targets, targets, sizeof(targets)));
     CK(cudaMemcpyToSymbol(dev::c_npos, npos, sizeof(npos)));
     CK(cudaMemcpyToSymbol(dev::c_nneg, nneg, sizeof(nneg)));
 }
