@@ -1020,6 +1020,13 @@ void run_coop(CoopPlan &P, int n, int every, bool skip_first, unsigned int *bar,
     }
 }
 
+bool is_capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cs));
+    return cs != cudaStreamCaptureStatusNone;
+}
+
 // A transport context steps by cooperative launches unless the caller chose a
 // plain-cell kernel (plain_path), the launch engine, or said that other contexts
 // share the GPU.
@@ -1027,7 +1034,11 @@ bool coop_ok(mgpu_ctx *ctx, bool residual)
 {
     if (ctx->adsorption || ctx->engine != MGPU_ENGINE_PERSISTENT || ctx->prm.plain_path >= 0 || ctx->prm.concurrent)
         return false;
-    if (!ctx->coop) ctx->coop = build_coop({ctx});
+    if (!ctx->coop)
+    {
+        if (is_capturing(ctx->stream)) return false; // nothing is allocated during a capture
+        ctx->coop = build_coop({ctx});
+    }
     return residual ? ctx->coop->ok_residual : ctx->coop->ok;
 }
 
@@ -1075,19 +1086,21 @@ void run_batch_with_residuals(mgpu_ctx *ctx, int n)
     if (n > 0 && coop_ok(ctx, true))
         run_coop(*ctx->coop, n, 1, true, ctx->grid_bar.p, ctx->stream, ctx->launches);
     else
-    for (int i = 0; i < n;)
     {
-        int64_t k = ctx->coarse_done + 1; // this step
-        bool diff = i > 0;                // residual of step k-1 (the previous batch closed its own last one)
-        if (diff && graphs && n - i >= 2 && !fresh_state(ctx))
+        for (int i = 0; i < n;)
         {
-            run_pair_graph(ctx, true, (int)((k - 1) % kRing));
-            i += 2;
-        }
-        else
-        {
-            coarse_step(ctx, diff, true, (int)(((k - 1) % kRing) * 4));
-            i++;
+            int64_t k = ctx->coarse_done + 1; // this step
+            bool diff = i > 0;                // residual of step k-1 (the previous batch closed its own last one)
+            if (diff && graphs && n - i >= 2 && !fresh_state(ctx))
+            {
+                run_pair_graph(ctx, true, (int)((k - 1) % kRing));
+                i += 2;
+            }
+            else
+            {
+                coarse_step(ctx, diff, true, (int)(((k - 1) % kRing) * 4));
+                i++;
+            }
         }
     }
     int64_t last = ctx->coarse_done;
@@ -2639,6 +2652,7 @@ bool batch_coop(mgpu_batch *b)
 {
     if (b->coop.empty())
     {
+        if (is_capturing(b->stream)) return false; // nothing is allocated during a capture
         int l2 = 0;
         CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, b->ctxs[0]->device));
         const int64_t most = 2 * (int64_t)l2;
