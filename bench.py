@@ -520,7 +520,7 @@ def run_properties(args):
                                "porosity 0.6, void x edges)", "thinning_iterations": int(iters)},
         "host_ms": round(1e3 * host_s, 1), "host_cores": 1,
         "bit_equal": bool(np.array_equal(lp, lp_h) and np.array_equal(kn, kn_h)),
-        "gpu_launches": 2 * 16 * int(-(-iters // 16)) + 9,
+        "gpu_launches": 8 * int(-(-iters // 128)) + 8,
     }))
 
 

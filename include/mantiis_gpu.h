@@ -121,9 +121,10 @@ int mgpu_run(mgpu_ctx *ctx, int n_steps, int *steps_done);
  * p->check_every steps into the history. */
 int mgpu_advance(mgpu_ctx *ctx, int n_steps);
 
-/* Same as mgpu_advance with no residual at all, replayed from a CUDA graph of
- * two coarse steps (captured on first use); enqueues the work and returns
- * without waiting.  The throughput path. */
+/* Same as mgpu_advance with no residual at all, in cooperative launches
+ * (mgpu_set_engine) or replayed from a CUDA graph of two coarse steps (captured
+ * on first use); enqueues the work and returns without waiting.  The throughput
+ * path. */
 int mgpu_advance_graph(mgpu_ctx *ctx, int n_steps);
 
 /* Profiling aid: enqueues n substeps of one level alone (the step kernel of
@@ -223,9 +224,10 @@ int64_t mgpu_launch_count(const mgpu_ctx *ctx);
 /* ---- batched stepping (no reference counterpart: the reference runs one
  * image per process, include/mantiisApp.hpp:286-430) ----
  * A batch steps a group of transport contexts of the current device together:
- * two coarse steps of every image are replayed from one CUDA graph in which the
- * images run on a few concurrent streams (as many as fit twice the L2 cache,
- * at least 2), so one image's small launches overlap another's work.  The
+ * groups of images in cooperative launches of many coarse steps, or two coarse
+ * steps of every image replayed from one CUDA graph in which the images run on a
+ * few concurrent streams (as many as fit twice the L2 cache, at least 2), so one
+ * image's small launches overlap another's work (mgpu_batch_set_engine).  The
  * contexts keep their state and stay usable on their own; batch work is
  * ordered after earlier work on each context's stream and before later work.
  * A context must not be stepped by two batches at once. */

@@ -315,7 +315,7 @@ class Solver:
         self._check(lib().mgpu_advance(self._h, int(n_steps)))
 
     def advance_graph(self, n_steps):
-        """Enqueues n coarse steps from a captured CUDA graph; returns without waiting."""
+        """Enqueues n coarse steps (mgpu_advance_graph); returns without waiting."""
         self._check(lib().mgpu_advance_graph(self._h, int(n_steps)))
 
     def set_engine(self, engine):
