@@ -2002,6 +2002,12 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
             for (size_t i = 0; i < pending.size(); i++) ctx->residuals.push_back(residual_of(ctx, &v[i * 4]));
             pending.clear();
         };
+        // before the slots of residuals first .. first + count - 1 are cleared or written:
+        // those still unread must not come around to them (with check_every = K they
+        // span K times as many slots as there are of them)
+        auto make_room = [&](int64_t first, int count) {
+            if (!pending.empty() && first + count - pending.front() > kRing) flush();
+        };
         // with a residual every step, pairs of steps replay a CUDA graph (not for
         // coupled runs, whose phase switch is host-side, nor from the initial state)
         auto pairs_ok = [&](int i) { return K == 1 && !ctx->coupled && n_steps - i >= 2 && !fresh_state(ctx); };
@@ -2019,6 +2025,7 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
                 {
                     // the rest of the call (as many steps as the pending slots hold) in one launch
                     const int m = std::min(n_steps - i, kRing / 2 - (int)pending.size());
+                    make_room(k, m);
                     zero_slots(ctx, (int)(k % kRing), m);
                     run_ads_persistent(ctx, m, k, true);
                     for (int j = 0; j < m; j++) pending.push_back(k + j);
@@ -2026,6 +2033,7 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
                 }
                 else if (pairs_ok(i))
                 {
+                    make_room(k, 2);
                     run_pair_graph(ctx, false, (int)(k % kRing));
                     pending.push_back(k);
                     pending.push_back(k + 1);
@@ -2034,7 +2042,11 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
                 else
                 {
                     bool diff = (k % K == 0);
-                    if (diff) zero_slots(ctx, (int)(k % kRing), 1);
+                    if (diff)
+                    {
+                        make_room(k, 1);
+                        zero_slots(ctx, (int)(k % kRing), 1);
+                    }
                     coarse_step(ctx, diff, false, (int)((k % kRing) * 4));
                     if (diff) pending.push_back(k);
                 }
@@ -2045,6 +2057,7 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
             {
                 // the rest of the call (as many steps as the pending slots hold) in one launch
                 const int m = std::min(n_steps - i, kRing / 2 - (int)pending.size());
+                make_room(k - 1, m);
                 zero_slots(ctx, (int)((k - 1) % kRing), m);
                 run_coop(*ctx->coop, m, K, false, ctx->grid_bar.p, ctx->stream, ctx->launches);
                 for (int64_t j = k; j < k + m; j++)
@@ -2058,6 +2071,7 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
             bool store = (k % K == 0);
             if (diff && pairs_ok(i))
             {
+                make_room(k - 1, 2);
                 run_pair_graph(ctx, true, (int)((k - 1) % kRing));
                 pending.push_back(k - 1);
                 pending.push_back(k);
@@ -2066,7 +2080,11 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
             else
             {
                 int slot = (int)(((k - 1) % kRing) * 4);
-                if (diff) zero_slots(ctx, (int)((k - 1) % kRing), 1);
+                if (diff)
+                {
+                    make_room(k - 1, 1);
+                    zero_slots(ctx, (int)((k - 1) % kRing), 1);
+                }
                 coarse_step(ctx, diff, store, slot);
                 if (diff) pending.push_back(k - 1);
             }
