@@ -23,6 +23,7 @@
 #include "../host/geometry.hpp"
 #include "../host/grid.hpp"
 #include "../host/units.hpp"
+#include "coop_groups.hpp"
 #include "kernels.cuh"
 #include "layout.hpp"
 
@@ -2676,25 +2677,12 @@ bool batch_coop(mgpu_batch *b)
         const int64_t most = 2 * (int64_t)l2;
         for (auto *c : b->ctxs)
             if (c->bytes > most) return false;
-        std::vector<mgpu_ctx *> group;
-        int64_t bytes = 0;
-        std::unique_ptr<CoopPlan> plan;
-        for (auto *c : b->ctxs)
-        {
-            group.push_back(c);
-            bytes += c->bytes;
-            std::unique_ptr<CoopPlan> more = build_coop(group);
-            if (plan && (bytes > most || !more->ok))
-            {
-                // the group ends before this image
-                b->coop.push_back(std::move(plan));
-                group = {c};
-                bytes = c->bytes;
-                more = build_coop(group);
-            }
-            plan = std::move(more);
-        }
-        b->coop.push_back(std::move(plan));
+        std::vector<int64_t> bytes;
+        for (auto *c : b->ctxs) bytes.push_back(c->bytes);
+        b->coop = coop_groups<CoopPlan>(bytes, most, [&](size_t first, size_t count) {
+            const auto at = b->ctxs.begin() + (std::ptrdiff_t)first;
+            return build_coop(std::vector<mgpu_ctx *>(at, at + (std::ptrdiff_t)count));
+        });
     }
     for (auto &g : b->coop)
         if (!g->ok) return false;
@@ -2825,8 +2813,11 @@ int mgpu_batch_advance(mgpu_batch *b, int n_steps)
         batch_enter(b);
         if (!b->engine_set && batch_coop(b))
         {
-            for (auto &g : b->coop) run_coop(*g, n_steps, 0, false, b->sync.p, b->stream, b->launches);
-            for (auto *c : b->ctxs) c->ref_t += n_steps;
+            for (auto &g : b->coop)
+            {
+                run_coop(*g, n_steps, 0, false, b->sync.p, b->stream, b->launches);
+                for (auto *c : g->ctxs) c->ref_t += n_steps;
+            }
             batch_leave(b);
             return MGPU_OK;
         }
