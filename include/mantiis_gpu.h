@@ -124,7 +124,12 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps);
 /* Same as mgpu_advance with no residual at all, in cooperative launches
  * (mgpu_set_engine) or replayed from a CUDA graph of two coarse steps (captured
  * on first use); enqueues the work and returns without waiting.  The throughput
- * path. */
+ * path.  Inside a caller's stream capture cooperative launches are recorded (once a
+ * call outside of one has made their plan): an even number of steps from a state that
+ * has been stepped, for any number of replays, or a single step, for one replay
+ * (further ones would start at the other parity); anything else is refused.  The
+ * context's step counts (mgpu_time) count the recording as one run of its steps, replays
+ * not at all. */
 int mgpu_advance_graph(mgpu_ctx *ctx, int n_steps);
 
 /* Profiling aid: enqueues n substeps of one level alone (the step kernel of

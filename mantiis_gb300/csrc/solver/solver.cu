@@ -1043,6 +1043,19 @@ bool coop_ok(mgpu_ctx *ctx, bool residual)
     return residual ? ctx->coop->ok_residual : ctx->coop->ok;
 }
 
+// Steps recorded by a caller's stream capture hold the parity of each level and
+// whether the state is the initial one as launch parameters.  Two steps or more
+// (which the launch engine's graph does not let be captured at all) are recorded
+// where every replay finds the state as the recording does; a single step is
+// recorded for one replay, as the launches per phase record it.
+void check_replayable(const mgpu_ctx *ctx, int n_steps)
+{
+    if (n_steps < 2 || !is_capturing(ctx->stream)) return;
+    for (size_t l = 0; l < ctx->lv.size(); l++)
+        if (ctx->lv[l].steps == 0 || ((int64_t)n_steps * ctx->lay.levels[l].substeps) % 2)
+            throw std::logic_error("steps inside a stream capture: an even number, from a state that has been stepped");
+}
+
 bool fresh_state(const mgpu_ctx *ctx)
 {
     for (auto &l : ctx->lv)
@@ -2110,6 +2123,7 @@ int mgpu_advance_graph(mgpu_ctx *ctx, int n_steps)
         }
         if (coop_ok(ctx, false))
         {
+            check_replayable(ctx, n_steps);
             run_coop(*ctx->coop, n_steps, 0, false, ctx->grid_bar.p, ctx->stream, ctx->launches);
             ctx->ref_t += n_steps;
             return MGPU_OK;
