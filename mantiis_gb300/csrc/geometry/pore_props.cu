@@ -26,6 +26,8 @@
 //      include/utils.hpp:116-135, visited in O(D) by nearest_skeleton_at),
 //      LocPore = 2 x its wall distance and Kn = mfp / LocPore / dx.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cfloat>
 #include <cstdint>
@@ -351,12 +353,20 @@ __global__ void k_local_pore(const int32_t *__restrict__ pore, BandSkeleton skel
 
 // The outputs are often fresh memory, whose pages the system gives out (and
 // clears) at the first write: that is done while the kernels run, not by the copy
-// that they end with.
-static void touch_pages(void *p, size_t bytes)
+// that they end with.  The system is asked for the pages, nothing is written here:
+// the outputs keep their content until the results arrive, and memory that it does
+// not manage (outputs on the GPU, pinned ones) is left alone.
+static void populate_pages(void *p, size_t bytes)
 {
-    volatile char *c = static_cast<volatile char *>(p);
-    for (size_t k = 0; k < bytes; k += 4096) c[k] = 0;
-    if (bytes) c[bytes - 1] = 0;
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), first = ((uintptr_t)p + page - 1) / page * page,
+                    end = ((uintptr_t)p + bytes) / page * page;
+    if (first < end)
+        (void)madvise(reinterpret_cast<void *>(first), end - first, MADV_POPULATE_WRITE); // refused: the copy does it
+#else
+    (void)p;
+    (void)bytes;
+#endif
 }
 
 void gpu_pore_properties(const int32_t *pore, int n, double dx, double mfp, double *locpore, double *kn,
@@ -409,8 +419,8 @@ void gpu_pore_properties(const int32_t *pore, int n, double dx, double mfp, doub
         GK(cudaGetLastError());
         if (done == 0)
         {
-            touch_pages(locpore, nn * sizeof(double));
-            touch_pages(kn, nn * sizeof(double));
+            populate_pages(locpore, nn * sizeof(double));
+            populate_pages(kn, nn * sizeof(double));
         }
         uint32_t host_flags[kLaunches];
         GK(cudaMemcpyAsync(host_flags, flags, sizeof(host_flags), cudaMemcpyDeviceToHost, stream));
