@@ -266,6 +266,12 @@ int mgpu_batch_set_engine(mgpu_batch *b, int engine, int group);
  * states.  A transport context uses engine 0 all the same where plain_path names a
  * kernel of it or `concurrent` says that other contexts share the GPU. */
 int mgpu_set_engine(mgpu_ctx *ctx, int engine);
+/* How often a block polls at a grid barrier of this context's cooperative launches
+ * (in a batch: of the group whose first image the context is) before it gives up:
+ * 0 (default) some seconds' worth.  Where a wait runs out, the launch ends and
+ * mgpu_sync of every image in it, mgpu_run and mgpu_batch_sync report MGPU_E_DEVICE;
+ * the states are then half stepped. */
+int mgpu_set_wait_limit(mgpu_ctx *ctx, uint32_t polls);
 int mgpu_batch_sync(mgpu_batch *b);
 int64_t mgpu_batch_launch_count(const mgpu_batch *b);
 int mgpu_batch_destroy(mgpu_batch *b);

@@ -1290,6 +1290,7 @@ struct AdsPersist
     int slot0, ring;        // residual of step k in slot (slot0 + k) mod ring
     int psi_diff;           // accumulate the residual of pass 1 (density change)
     unsigned int *bar;      // arrivals at the grid barriers; zero at launch
+    uint32_t polls;         // of a barrier's wait before the block gives up
 };
 
 // shared memory of one warp of cells: this many floats per lane
@@ -1337,13 +1338,14 @@ __device__ __forceinline__ void add_block_sums(const double2 *sums, double *dst)
 
 // Grid barrier `target` = (barriers passed) x gridDim.x: every block adds one
 // arrival with release semantics after its block barrier, then waits (bounded)
-// for all of them; a wait that runs out sets the error word and the block stops.
+// for all of them, at most `polls` polls; where they run out (false) the caller
+// notes it in the error word and the block stops.
 // rmax: if not null, the block's maximum of the residual terms (non-negative
 // floats by their bit patterns), which goes to dst and is cleared; clear: a
 // counter in shared memory set to zero on the way; sums: if not null, the warps'
 // pairs of sums in shared memory (block_sums), which warp 1 adds to sums_to while
 // the block waits.
-__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int target, unsigned int *err,
+__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int target, uint32_t polls,
                                              unsigned int *rmax, double *dst, unsigned int *clear = nullptr,
                                              const double2 *sums = nullptr, double *sums_to = nullptr)
 {
@@ -1361,13 +1363,12 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int tar
         if (clear) *clear = 0u;
         add_release(bar, 1u);
         bool ok = false;
-        for (uint32_t i = 0; i < kDepPolls && !ok; i++)
+        for (uint32_t i = 0; i < polls && !ok; i++)
         {
             unsigned int v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             ok = v >= target;
         }
-        if (!ok) atomicOr(err, kErrDepTimeout);
         s_ok = ok ? 1 : 0;
     }
     __syncthreads();
@@ -1655,13 +1656,20 @@ __global__ void __launch_bounds__(THREADS, 1) k_ads_persistent(const __grid_cons
             if ((threadIdx.x & 31) == 0 && v) atomicMax(&s_rmax, v);
         }
         target += gridDim.x;
-        if (!grid_barrier(A.bar, target, A.C.err, A.psi_diff ? &s_rmax : nullptr,
+        if (!grid_barrier(A.bar, target, A.polls, A.psi_diff ? &s_rmax : nullptr,
                           A.C.red + (size_t)((A.slot0 + k) % A.ring) * 4))
+        {
+            if (threadIdx.x == 0) atomicOr(A.C.err, kErrDepTimeout);
             return;
+        }
         if (parity) ads_pass2<1, FITS>(A, B, sm, o, direct);
         else ads_pass2<0, FITS>(A, B, sm, o, direct);
         target += gridDim.x;
-        if (!last && !grid_barrier(A.bar, target, A.C.err, nullptr, nullptr)) return;
+        if (!last && !grid_barrier(A.bar, target, A.polls, nullptr, nullptr))
+        {
+            if (threadIdx.x == 0) atomicOr(A.C.err, kErrDepTimeout);
+            return;
+        }
     }
 }
 
@@ -1730,7 +1738,8 @@ struct CoopLaunch
     // ring; skip_first: not by the launch's first step, whose number mod `every` is
     // since0 and whose predecessor's slot is slot0
     int every, skip_first, ring, since0, slot0;
-    unsigned int *bar, *err; // grid-barrier arrivals (zero at launch), error word
+    unsigned int *bar; // grid-barrier arrivals; zero at launch
+    uint32_t polls;    // of a barrier's wait before the block gives up
     CoopDesc d[kMaxCoopDescs];
     CoopPair p[kMaxCoopPairs];
 };
@@ -2225,6 +2234,12 @@ __device__ __forceinline__ void coop_cells(const CoopLaunch &A, const CoopRange 
     }
 }
 
+// a barrier's wait ran out: every image of the launch is left half stepped
+__device__ __forceinline__ void coop_gave_up(const CoopLaunch &A)
+{
+    for (int d = (int)threadIdx.x; d < A.nd; d += (int)blockDim.x) atomicOr(A.d[d].C.err, kErrDepTimeout);
+}
+
 // DEF: every image has the default regularized MRT and SRBB walls (their code
 // alone then passes through the instruction cache); RES: with residuals (A.every)
 template <int THREADS, bool DEF, bool RES>
@@ -2330,7 +2345,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_coop_steps(const __grid_constant
                 if (!end)
                 {
                     target += gridDim.x;
-                    if (!grid_barrier(A.bar, target, A.err, nullptr, nullptr, &s_next, s_sums, red)) return;
+                    if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next, s_sums, red)) return coop_gave_up(A);
                     continue;
                 }
                 __syncthreads();
@@ -2338,7 +2353,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_coop_steps(const __grid_constant
             }
             if (end) break;
             target += gridDim.x;
-            if (!grid_barrier(A.bar, target, A.err, nullptr, nullptr, &s_next)) return;
+            if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next)) return coop_gave_up(A);
         }
 #pragma unroll 1
         for (int w = 0; w < A.nwave; w++)
@@ -2381,7 +2396,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_coop_steps(const __grid_constant
             }
             if (k + 1 == A.nsteps && w + 1 == A.nwave) break;
             target += gridDim.x;
-            if (!grid_barrier(A.bar, target, A.err, nullptr, nullptr, &s_next)) return;
+            if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next)) return coop_gave_up(A);
         }
     }
     if (RES)

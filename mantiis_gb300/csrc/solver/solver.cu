@@ -277,6 +277,7 @@ struct mgpu_ctx
     // steps replayed from a CUDA graph)
     int engine = MGPU_ENGINE_PERSISTENT;
     DevBuf<unsigned int> grid_bar; // grid-barrier arrivals of the cooperative launches
+    uint32_t wait_polls = dev::kDepPolls; // of a grid barrier's wait (mgpu_set_wait_limit)
     std::unique_ptr<CoopPlan> coop; // cooperative transport launch of this image
     float rho0f = 0.f;
     bool adsorption = false; // Shan-Chen step body (include/mantiisApp.hpp:248-265)
@@ -517,7 +518,8 @@ void check_device_error(mgpu_ctx *ctx)
     {
         CK(cudaMemsetAsync(ctx->errword.p, 0, sizeof(w), ctx->stream));
         throw DeviceError("device error flag " + std::to_string(w) +
-                          ((w & dev::kErrTmaTimeout) ? ": a tile copy did not complete in time" : ""));
+                          ((w & dev::kErrTmaTimeout) ? ": a tile copy did not complete in time" : "") +
+                          ((w & dev::kErrDepTimeout) ? ": a wait for other blocks ran out; the state is half stepped" : ""));
     }
 }
 
@@ -838,6 +840,7 @@ void run_ads_persistent(mgpu_ctx *ctx, int n, int64_t k, bool diff)
     A.ring = kRing;
     A.psi_diff = diff ? 1 : 0; // the density change (the coupling phase, with |u| sums, is not run here)
     A.bar = ctx->grid_bar.p;
+    A.polls = ctx->wait_polls;
     // one block per SM with at least four warps of cells each; the warps of a
     // block share its warps of cells evenly, as much of their data as fits in
     // shared memory
@@ -1000,7 +1003,7 @@ void run_coop(CoopPlan &P, int n, int every, bool skip_first, unsigned int *bar,
         A.since0 = every ? (int)(k0 % every) : 0;
         A.slot0 = (int)((k0 - 1) % kRing);
         A.bar = bar;
-        A.err = P.ctxs[0]->errword.p;
+        A.polls = P.ctxs[0]->wait_polls;
         int d = 0;
         for (auto *c : P.ctxs)
             for (auto &l : c->lv)
@@ -2205,6 +2208,15 @@ int mgpu_set_engine(mgpu_ctx *ctx, int engine)
     });
 }
 
+int mgpu_set_wait_limit(mgpu_ctx *ctx, uint32_t polls)
+{
+    return guarded(ctx, [&]() {
+        if (!ctx) throw std::invalid_argument("null context");
+        ctx->wait_polls = polls ? polls : dev::kDepPolls;
+        return MGPU_OK;
+    });
+}
+
 int mgpu_step_level(mgpu_ctx *ctx, int level, int n)
 {
     return guarded(ctx, [&]() {
@@ -2982,7 +2994,18 @@ int mgpu_batch_sync(mgpu_batch *b)
     return guarded(nullptr, [&]() {
         if (!b) throw std::invalid_argument("null batch");
         CK(cudaStreamSynchronize(b->stream));
-        for (auto *c : b->ctxs) check_device_error(c);
+        // every image's word is read (and cleared) before the first error is reported
+        std::string error;
+        for (auto *c : b->ctxs)
+            try
+            {
+                check_device_error(c);
+            }
+            catch (const DeviceError &e)
+            {
+                if (error.empty()) error = e.what();
+            }
+        if (!error.empty()) throw DeviceError(error);
         return MGPU_OK;
     });
 }

@@ -106,6 +106,7 @@ SIGNATURES = {
     "mgpu_batch_set_stream": (C.c_int, [P, P]),
     "mgpu_batch_set_engine": (C.c_int, [P, C.c_int, C.c_int]),
     "mgpu_set_engine": (C.c_int, [P, C.c_int]),
+    "mgpu_set_wait_limit": (C.c_int, [P, C.c_uint32]),
     "mgpu_batch_sync": (C.c_int, [P]),
     "mgpu_batch_launch_count": (C.c_int64, [P]),
     "mgpu_batch_destroy": (C.c_int, [P]),
