@@ -300,6 +300,7 @@ struct mgpu_ctx
     std::unique_ptr<PhasePlan> plan; // phase engine tables of this image
     std::vector<std::unique_ptr<PhasePlan>> level_plans; // single-level tables (mgpu_step_level)
     int sm_count = 1;
+    int stream_sms = 1; // of these, what kernels on `stream` can use
     double autotune_us[3] = {0.0, 0.0, 0.0}; // plain_path -1: microseconds per coarse step of paths 0, 1, 2
     int64_t coarse_done = 0;     // coarse steps executed since creation
     int64_t ref_t = 0;           // reference lb->t
@@ -457,6 +458,31 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
         fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
     }
     return fn;
+}
+
+// SMs that kernels on a stream can use: those of the device, or of the part of it
+// that the stream's context was given (a green context), at least one.  A stream
+// keeps its part for life.
+int sms_of_stream(cudaStream_t stream, int device_sms)
+{
+    static const auto entry = [](const char *name, unsigned version) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion(name, &p, version, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        cudaGetLastError();
+        return p;
+    };
+    static const auto get_ctx = reinterpret_cast<PFN_cuStreamGetCtx_v9020>(entry("cuStreamGetCtx", 9020));
+    static const auto get_part = reinterpret_cast<PFN_cuCtxGetDevResource_v12040>(entry("cuCtxGetDevResource", 12040));
+    CUcontext c = nullptr;
+    CUdevResource part;
+    std::memset(&part, 0, sizeof(part));
+    if (!get_ctx || !get_part || get_ctx((CUstream)stream, &c) != CUDA_SUCCESS ||
+        get_part(c, &part, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+        return device_sms;
+    return std::max(1, std::min(device_sms, (int)part.sm.smCount));
 }
 
 // the level's 9 planes as a 3-D tensor (x: pitch floats, y: H rows, q: 9
@@ -845,7 +871,7 @@ void run_ads_persistent(mgpu_ctx *ctx, int n, int64_t k, bool diff)
     // block share its warps of cells evenly, as much of their data as fits in
     // shared memory
     const int warps = (A.nplain + 31) / 32 + (A.spec_count + 31) / 32;
-    const int grid = std::max(1, std::min(ctx->sm_count, warps / 4));
+    const int grid = std::max(1, std::min(ctx->stream_sms, warps / 4));
     const int ws = (A.spec_count / grid + 32) / 32, wp = (A.nplain / grid + 32) / 32, per_block = ws + wp;
     const bool small = per_block * 32 <= dev::kAdsSmall;
     const int most = (small ? dev::kAdsSmall : dev::kAdsLarge) / 32;
@@ -981,7 +1007,16 @@ std::unique_ptr<CoopPlan> build_coop(const std::vector<mgpu_ctx *> &ctxs)
     P->kernel[1] = P->def ? (const void *)dev::k_coop_steps<kCoopResThreads, true, true>
                           : (const void *)dev::k_coop_steps<kCoopResThreads, false, true>;
     for (const void *k : P->kernel) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
-    P->ok = true;
+    // (every block resident: one per SM)
+    for (int res = 0; res < 2; res++)
+    {
+        if (res && !P->ok_residual) break;
+        int per_sm = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, P->kernel[res], P->threads[res], P->smem[res]));
+        if (res) P->ok_residual = per_sm >= 1;
+        else P->ok = per_sm >= 1;
+    }
+    P->ok_residual = P->ok_residual && P->ok;
     return P;
 }
 
@@ -1033,7 +1068,9 @@ bool is_capturing(cudaStream_t s)
 
 // A transport context steps by cooperative launches unless the caller chose a
 // plain-cell kernel (plain_path), the launch engine, or said that other contexts
-// share the GPU.
+// share the GPU.  Its blocks are one per SM of the device (the shares of the cells
+// are made for them) and must be resident together: a stream of fewer SMs takes
+// the launches.
 bool coop_ok(mgpu_ctx *ctx, bool residual)
 {
     if (ctx->adsorption || ctx->engine != MGPU_ENGINE_PERSISTENT || ctx->prm.plain_path >= 0 || ctx->prm.concurrent)
@@ -1043,7 +1080,7 @@ bool coop_ok(mgpu_ctx *ctx, bool residual)
         if (is_capturing(ctx->stream)) return false; // nothing is allocated during a capture
         ctx->coop = build_coop({ctx});
     }
-    return residual ? ctx->coop->ok_residual : ctx->coop->ok;
+    return ctx->coop->grid <= ctx->stream_sms && (residual ? ctx->coop->ok_residual : ctx->coop->ok);
 }
 
 // Steps recorded by a caller's stream capture hold the parity of each level and
@@ -1755,6 +1792,7 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
     CK(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device));
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     ctx->own_stream = true;
+    ctx->stream_sms = sms_of_stream(ctx->stream, ctx->sm_count);
     ctx->lanes.create();
     upload_constants();
     cudaStream_t s = ctx->stream;
@@ -2620,6 +2658,7 @@ int mgpu_set_stream(mgpu_ctx *ctx, void *stream)
             CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
             ctx->own_stream = true;
         }
+        ctx->stream_sms = sms_of_stream(ctx->stream, ctx->sm_count);
         return MGPU_OK;
     });
 }
@@ -2663,7 +2702,7 @@ struct mgpu_batch
     std::map<std::string, std::unique_ptr<PersistPlan>> pplans;
     DevBuf<unsigned int> sync; // claim and stage counters of the persistent launch
     int64_t bytes = 0;
-    int sm_count = 1;
+    int sm_count = 1, stream_sms = 1;
 };
 
 namespace
@@ -2711,7 +2750,7 @@ bool batch_coop(mgpu_batch *b)
         });
     }
     for (auto &g : b->coop)
-        if (!g->ok) return false;
+        if (!g->ok || g->grid > b->stream_sms) return false;
     return true;
 }
 
@@ -2824,6 +2863,7 @@ int mgpu_batch_create(mgpu_ctx *const *ctxs, int n, mgpu_batch **out)
         b->ctx_ev.resize(b->ctxs.size());
         for (auto &e : b->ctx_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         b->sm_count = b->ctxs[0]->sm_count;
+        b->stream_sms = sms_of_stream(b->stream, b->sm_count);
         // stage counters of two coarse steps: at most 2^(L-1) phases and L waves
         // per image and step (L <= 4)
         b->sync.alloc(1 + b->ctxs.size() * 2 * (8 + 4), b->bytes);
@@ -2985,6 +3025,7 @@ int mgpu_batch_set_stream(mgpu_batch *b, void *stream)
             CK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
             b->own_stream = true;
         }
+        b->stream_sms = sms_of_stream(b->stream, b->sm_count);
         return MGPU_OK;
     });
 }
