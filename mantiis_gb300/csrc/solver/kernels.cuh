@@ -537,8 +537,11 @@ __global__ void __launch_bounds__(256, 4) k_phase_plain_tma(const __grid_constan
         const int diff = P.a.diff & d.o.first_sub, store_u = P.a.store_u & d.o.first_sub;
         if (diff) red_desc = j;
         const int tile = s_tile[st];
-        if (d.o.parity) plain_tile_smem<1>(d.L, d.C, d.o, tile, sbuf[st], diff, store_u, r_diff, r_norm);
-        else plain_tile_smem<0>(d.L, d.C, d.o, tile, sbuf[st], diff, store_u, r_diff, r_norm);
+        double t_diff = 0.0, t_norm = 0.0; // this tile's terms
+        if (d.o.parity) plain_tile_smem<1>(d.L, d.C, d.o, tile, sbuf[st], diff, store_u, t_diff, t_norm);
+        else plain_tile_smem<0>(d.L, d.C, d.o, tile, sbuf[st], diff, store_u, t_diff, t_norm);
+        r_diff += t_diff;
+        r_norm += t_norm;
         // every thread is done with this stage before it is refilled
         __syncthreads();
         if (threadIdx.x == 0)
