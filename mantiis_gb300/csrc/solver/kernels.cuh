@@ -1366,7 +1366,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int tar
         if (clear) *clear = 0u;
         add_release(bar, 1u);
         bool ok = false;
-        for (uint32_t i = 0; i < polls && !ok; i++)
+        for (uint32_t i = polls; i != 0 && !ok; i--)
         {
             unsigned int v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
@@ -1741,7 +1741,7 @@ struct CoopLaunch
     // ring; skip_first: not by the launch's first step, whose number mod `every` is
     // since0 and whose predecessor's slot is slot0
     int every, skip_first, ring, since0, slot0;
-    unsigned int *bar; // grid-barrier arrivals; zero at launch
+    unsigned int *bar; // grid-barrier arrivals, blocks that have left; both zero at launch and after it
     uint32_t polls;    // of a barrier's wait before the block gives up
     CoopDesc d[kMaxCoopDescs];
     CoopPair p[kMaxCoopPairs];
@@ -1768,10 +1768,11 @@ __device__ __forceinline__ uint32_t coop_site(const LevelView &L, int x, int y)
            (y == 0 ? kCoopLow : 0u) | (y + 1 == L.H ? kCoopHigh : 0u);
 }
 
-struct CoopRange // a block's cells of one kind and level, or rows (lo in warps)
+struct CoopRange // a block's cells of one kind and level, or rows (lo in warps, 32 "cells" to a warp)
 {
     int lo, cells; // first cell, cells
-    int n, line;   // warps of cells or rows, first line
+    int n, line;   // warps of cells or rows, first line; coop_place: n of the ranges before
+    __device__ __forceinline__ int warps() const { return (cells + 31) >> 5; }
 };
 
 // Slots of a cell.  A step reads and writes the same nine: on plane p its own
@@ -2188,59 +2189,159 @@ __device__ __forceinline__ void coop_fine(const CoopSide &F, const CoopSide &Cd,
     if (buf & kCoopBuf) CoopSlots(F.L, F.stride, at, F.par).fill(acc);
 }
 
-// fills the block's shared memory (BACK false), or writes the stored |u| back
+// First line of each of `count` ranges, whose lines start at `line`, and (in n) the
+// number of warps before it; returns the line after them.  One warp, 32 ranges at a time.
+template <typename Lines>
+__device__ __forceinline__ int coop_place(CoopRange *rng, int count, int line, Lines lines_of)
+{
+    const int lane = threadIdx.x & 31;
+    int all = 0;
+    for (int t0 = 0; t0 < count; t0 += 32)
+    {
+        const int t = t0 + lane, n = t < count ? rng[t].warps() : 0, own = t < count ? n * lines_of(t) : 0;
+        int sn = n, sl = own; // sums up to and with this lane
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int un = __shfl_up_sync(0xffffffffu, sn, o), ul = __shfl_up_sync(0xffffffffu, sl, o);
+            if (lane >= o) sn += un, sl += ul;
+        }
+        if (t < count)
+        {
+            rng[t].line = line + sl - own;
+            rng[t].n = all + sn - n;
+        }
+        all += __shfl_sync(0xffffffffu, sn, 31);
+        line += __shfl_sync(0xffffffffu, sl, 31);
+    }
+    return line;
+}
+
+// The block's warps of cells (or rows) of all ranges, numbered through: warp w takes
+// w, w + nw, ...; find() advances to the range of one.
+struct CoopItems
+{
+    const CoopRange *rng;
+    int count, total, t;
+    __device__ __forceinline__ CoopItems(const CoopRange *r, int n)
+        : rng(r), count(n), total(n ? r[n - 1].n + r[n - 1].warps() : 0), t(0)
+    {
+    }
+    __device__ __forceinline__ void find(int i)
+    {
+        while (t + 1 < count && i >= rng[t + 1].n) t++;
+    }
+};
+
+// Fills the block's shared memory (BACK false), or writes the stored |u| back.  A
+// warp has kCoopFill warps of cells in flight, of whichever image, level and kind: a
+// launch pays a few round trips to memory for it.  (List by list, one warp of cells at
+// a time, a call of one step of eight 512^2 images of two levels took 345 us; now 301.)
 template <bool BACK, bool RES>
 __device__ __forceinline__ void coop_cells(const CoopLaunch &A, const CoopRange *rng, float *sm)
 {
+    constexpr int kCoopFill = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int d = 0; d < A.nd; d++)
+    CoopItems items(rng, A.nd * CK_KINDS);
+#pragma unroll 1
+    for (int i0 = warp; i0 < items.total; i0 += kCoopFill * nw)
     {
-        const CoopDesc &D = A.d[d];
-        for (int kind = 0; kind < CK_KINDS; kind++)
+        int at[kCoopFill], xy[kCoopFill]; // range, position; -1: none
+        float *m[kCoopFill];
+#pragma unroll
+        for (int u = 0; u < kCoopFill; u++)
         {
-            const CoopRange r = rng[d * CK_KINDS + kind];
-            for (int i = warp; i < r.n; i += nw)
+            const int i = i0 + u * nw;
+            at[u] = xy[u] = -1;
+            if (i >= items.total) continue;
+            items.find(i);
+            const CoopRange &r = rng[items.t];
+            const CoopDesc &D = A.d[items.t / CK_KINDS];
+            const int kind = items.t % CK_KINDS, k = i - r.n, c = r.lo + k * 32 + lane;
+            at[u] = items.t;
+            m[u] = sm + (size_t)(r.line + k * D.lines[kind]) * 32;
+            if (k * 32 + lane >= r.cells) continue;
+            if (kind >= CK_EDGE) xy[u] = __ldg(&D.xy[kind][c]);
+            else
             {
-                const int c = r.lo + i * 32 + lane;
-                const bool there = i * 32 + lane < r.cells;
-                float *m = sm + (size_t)(r.line + i * D.lines[kind]) * 32;
-                float *un = m + (kind >= CK_EDGE ? 2 : 8) * 32 + lane;
-                int xy = -1;
-                if (kind >= CK_EDGE)
+                const SpecialRec *rec = D.C.specials + D.spec_begin + (kind == CK_LIGHT ? D.nheavy : 0) + c;
+                if (BACK) xy[u] = rec->xy;
+                else
                 {
-                    if (there) xy = __ldg(&D.xy[kind][c]);
-                    if (!BACK)
-                    {
-                        const uint32_t site = there ? coop_site(D.L, xy & 0xFFFF, xy >> 16) : kCoopNone;
-                        m[lane] = __uint_as_float(site);
-                        if (there) m[32 + lane] = D.L.omega[site & kCoopSite];
-                    }
+                    const uint4 r0 = reinterpret_cast<const uint4 *>(rec)[0], r1 = reinterpret_cast<const uint4 *>(rec)[1];
+                    reinterpret_cast<uint4 *>(m[u])[lane] = r0;
+                    reinterpret_cast<uint4 *>(m[u])[32 + lane] = r1;
+                    xy[u] = (int)r1.z;
                 }
-                else if (there)
-                {
-                    const uint4 *rec = reinterpret_cast<const uint4 *>(D.C.specials + D.spec_begin +
-                                                                       (kind == CK_LIGHT ? D.nheavy : 0) + c);
-                    const uint4 r0 = rec[0], r1 = rec[1];
-                    xy = (int)r1.z;
-                    if (!BACK)
-                    {
-                        reinterpret_cast<uint4 *>(m)[lane] = r0;
-                        reinterpret_cast<uint4 *>(m)[32 + lane] = r1;
-                    }
-                }
-                if (!there || !RES) continue;
-                float *g = &D.L.unorm[site_of(D.L, xy & 0xFFFF, xy >> 16)];
-                if (BACK) *g = *un;
-                else *un = *g;
             }
+        }
+#pragma unroll
+        for (int u = 0; u < kCoopFill; u++)
+        {
+            if (at[u] < 0) continue;
+            const CoopDesc &D = A.d[at[u] / CK_KINDS];
+            const int kind = at[u] % CK_KINDS;
+            const bool there = xy[u] >= 0;
+            if (!BACK && kind >= CK_EDGE)
+            {
+                const uint32_t site = there ? coop_site(D.L, xy[u] & 0xFFFF, xy[u] >> 16) : kCoopNone;
+                m[u][lane] = __uint_as_float(site);
+                if (there) m[u][32 + lane] = D.L.omega[site & kCoopSite];
+            }
+            if (!there || !RES) continue;
+            float *un = m[u] + (kind >= CK_EDGE ? 2 : 8) * 32 + lane;
+            float *g = &D.L.unorm[site_of(D.L, xy[u] & 0xFFFF, xy[u] >> 16)];
+            if (BACK) *g = *un;
+            else *un = *g;
         }
     }
 }
 
-// a barrier's wait ran out: every image of the launch is left half stepped
-__device__ __forceinline__ void coop_gave_up(const CoopLaunch &A)
+__device__ __forceinline__ int coop_place_cells(const CoopLaunch &A, CoopRange *rng)
 {
-    for (int d = (int)threadIdx.x; d < A.nd; d += (int)blockDim.x) atomicOr(A.d[d].C.err, kErrDepTimeout);
+    return coop_place(rng, A.nd * CK_KINDS, 0, [&](int t) { return A.d[t / CK_KINDS].lines[t % CK_KINDS]; });
+}
+
+// The places of a block's lists in shared memory, and their content.  (A call: inlined,
+// it cost the stages' loops up to 0.6 % by the registers and places they got.)
+template <bool RES>
+__device__ __noinline__ void coop_start(const CoopLaunch &A, CoopRange *rng, CoopRange *rows, unsigned int *next, float *sm)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (warp == 0)
+    {
+        if (lane == 0) *next = 0u;
+        const int line = coop_place_cells(A, rng);
+        coop_place(rows, A.np * 2, line, [](int t) { return t & 1 ? kCoopFineLines : kCoopCoarseLines; });
+    }
+    __syncthreads();
+    coop_cells<false, RES>(A, rng, sm);
+    CoopItems waves(rows, A.np * 2);
+    for (int i = warp; i < waves.total; i += nw)
+    {
+        waves.find(i);
+        const int t = waves.t, k = i - rows[t].n, r = (rows[t].lo + k) * 8 + lane / 4;
+        const CoopPair &Q = A.p[t / 2];
+        const LevelView &Lf = A.d[Q.df].L, &Lc = A.d[Q.dc].L;
+        if (t & 1) coop_fill_fine(Q, Lf, Lc, r, lane & 3, sm + (size_t)(rows[t].line + k * kCoopFineLines) * 32);
+        else coop_fill_coarse(Q, Lf, Lc, r, lane & 3, sm + (size_t)(rows[t].line + k * kCoopCoarseLines) * 32);
+    }
+    __syncthreads();
+    for (int t = (int)threadIdx.x; t < A.nd * CK_KINDS; t += (int)blockDim.x) rng[t].n = rng[t].warps();
+    for (int t = (int)threadIdx.x; t < A.np * 2; t += (int)blockDim.x) rows[t].n = rows[t].warps();
+}
+
+// The block has passed its last barrier: the last block to come here clears the
+// counters for the next launch (a memset before each launch took as long as half a
+// step of a small image).  Where a barrier's wait ran out (!ok), every image of the
+// launch is left half stepped and noted so.
+__device__ __forceinline__ void coop_leave(const CoopLaunch &A, bool ok)
+{
+    if (!ok)
+        for (int d = (int)threadIdx.x; d < A.nd; d += (int)blockDim.x) atomicOr(A.d[d].C.err, kErrDepTimeout);
+    if (threadIdx.x != 0) return;
+    __threadfence(); // this block's arrivals come before its leave
+    if (atomicAdd(A.bar + 1, 1u) + 1u == gridDim.x) A.bar[0] = A.bar[1] = 0u;
 }
 
 // DEF: every image has the default regularized MRT and SRBB walls (their code
@@ -2263,7 +2364,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_coop_steps(const __grid_constant
         const int32_t *cut = A.d[t / CK_KINDS].cut[t % CK_KINDS];
         rng[t].lo = cut[b];
         rng[t].cells = cut[b + 1] - rng[t].lo;
-        rng[t].n = (rng[t].cells + 31) / 32;
     }
     for (int t = (int)threadIdx.x; t < A.nd; t += (int)blockDim.x)
         strides[t] = make_uint2((uint32_t)A.d[t].L.plane, (uint32_t)A.d[t].L.pitch);
@@ -2272,139 +2372,120 @@ __global__ void __launch_bounds__(THREADS, 1) k_coop_steps(const __grid_constant
         const CoopPair &Q = A.p[t / 2];
         const int W = ((t & 1 ? Q.nfine : Q.ncoarse) + 7) / 8;
         rows[t].lo = coop_cut(W, Q.rot, b, G);
-        rows[t].n = coop_cut(W, Q.rot, b + 1, G) - rows[t].lo;
+        rows[t].cells = (coop_cut(W, Q.rot, b + 1, G) - rows[t].lo) * 32;
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        s_next = 0u;
-        int line = 0;
-        for (int t = 0; t < A.nd * CK_KINDS; t++)
-        {
-            rng[t].line = line;
-            line += rng[t].n * A.d[t / CK_KINDS].lines[t % CK_KINDS];
-        }
-        for (int t = 0; t < A.np * 2; t++)
-        {
-            rows[t].line = line;
-            line += rows[t].n * (t & 1 ? kCoopFineLines : kCoopCoarseLines);
-        }
-    }
+    coop_start<RES>(A, rng, rows, &s_next, sm);
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    coop_cells<false, RES>(A, rng, sm);
-    for (int t = 0; t < A.np * 2; t++)
-    {
-        const CoopPair &Q = A.p[t / 2];
-        const LevelView &Lf = A.d[Q.df].L, &Lc = A.d[Q.dc].L;
-        for (int i = warp; i < rows[t].n; i += nw)
-        {
-            const int r = (rows[t].lo + i) * 8 + lane / 4;
-            if (t & 1) coop_fill_fine(Q, Lf, Lc, r, lane & 3, sm + (size_t)(rows[t].line + i * kCoopFineLines) * 32);
-            else coop_fill_coarse(Q, Lf, Lc, r, lane & 3, sm + (size_t)(rows[t].line + i * kCoopCoarseLines) * 32);
-        }
-    }
-    __syncthreads();
-    unsigned int target = 0;
-    int since = A.since0, prev = since == 0 ? A.every - 1 : since - 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // every step; false where a barrier's wait ran out
+    auto steps = [&]() -> bool {
+        unsigned int target = 0;
+        int since = A.since0, prev = since == 0 ? A.every - 1 : since - 1;
 #pragma unroll 1
-    for (int k = 0; k < A.nsteps; k++)
-    {
-        const bool store = RES && since == 0; // this step's number is a multiple of A.every
-        const bool diff = RES && prev == 0 && !(k == 0 && A.skip_first);
-        if (RES)
+        for (int k = 0; k < A.nsteps; k++)
         {
-            prev = since;
-            since = since + 1 == A.every ? 0 : since + 1;
-        }
-#pragma unroll 1
-        for (int ph = 0; ph < A.nphase; ph++)
-        {
-            CoopClaim claim(&s_next);
-            if (RES && diff && ph == 0) *acc = make_double2(0.0, 0.0);
-#pragma unroll 1
-            for (int d = 0; d < A.nd; d++)
+            const bool store = RES && since == 0; // this step's number is a multiple of A.every
+            const bool diff = RES && prev == 0 && !(k == 0 && A.skip_first);
+            if (RES)
             {
-                const CoopDesc &D = A.d[d];
-                if (ph & ((1 << D.shift) - 1)) continue;
-                const int sub = ph >> D.shift;
-                CoopStep st{};
-                st.o.parity = (D.parity0 + k * D.substeps + sub) & 1;
-                st.o.direct = k == 0 && sub == 0 && D.direct0;
-                st.o.first_sub = sub == 0;
-                st.o.snap_store = D.mb && sub == 0;
-                st.o.snap_use = D.mb && sub > 0;
-                st.diff = diff && sub == 0;
-                st.store_u = store && sub == 0;
-                st.collision = DEF ? COLL_RMRT : D.C.collision;
-                st.wall = DEF ? WALL_SRBB : D.C.wall;
-                coop_level<RES>(A, d, st, rng + d * CK_KINDS, strides + d, sm, claim, acc);
+                prev = since;
+                since = since + 1 == A.every ? 0 : since + 1;
             }
-            if (RES && diff && ph == 0) block_sums(acc->x, acc->y, s_sums);
-            const bool end = k + 1 == A.nsteps && ph + 1 == A.nphase && A.nwave == 0;
-            if (RES && diff && ph == 0)
+#pragma unroll 1
+            for (int ph = 0; ph < A.nphase; ph++)
             {
-                double *red = A.d[0].C.red + (size_t)((uint32_t)(A.slot0 + k) % (uint32_t)A.ring) * 4;
-                if (!end)
+                CoopClaim claim(&s_next);
+                if (RES && diff && ph == 0) *acc = make_double2(0.0, 0.0);
+#pragma unroll 1
+                for (int d = 0; d < A.nd; d++)
                 {
-                    target += gridDim.x;
-                    if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next, s_sums, red)) return coop_gave_up(A);
-                    continue;
+                    const CoopDesc &D = A.d[d];
+                    if (ph & ((1 << D.shift) - 1)) continue;
+                    const int sub = ph >> D.shift;
+                    CoopStep st{};
+                    st.o.parity = (D.parity0 + k * D.substeps + sub) & 1;
+                    st.o.direct = k == 0 && sub == 0 && D.direct0;
+                    st.o.first_sub = sub == 0;
+                    st.o.snap_store = D.mb && sub == 0;
+                    st.o.snap_use = D.mb && sub > 0;
+                    st.diff = diff && sub == 0;
+                    st.store_u = store && sub == 0;
+                    st.collision = DEF ? COLL_RMRT : D.C.collision;
+                    st.wall = DEF ? WALL_SRBB : D.C.wall;
+                    coop_level<RES>(A, d, st, rng + d * CK_KINDS, strides + d, sm, claim, acc);
                 }
-                __syncthreads();
-                if (warp == 1) add_block_sums(s_sums, red);
-            }
-            if (end) break;
-            target += gridDim.x;
-            if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next)) return coop_gave_up(A);
-        }
-#pragma unroll 1
-        for (int w = 0; w < A.nwave; w++)
-        {
-            CoopClaim claim(&s_next);
-#pragma unroll 1
-            for (int p = 0; p < A.np; p++)
-            {
-                const CoopPair &Q = A.p[p];
-                const int kind = Q.l1 - 1 == w ? 0 : Q.l1 == w ? 1 : -1; // coarse rows / fine rows
-                if (kind < 0) continue;
-                const CoopRange rr = rows[p * 2 + kind];
-                const int nrows = kind == 0 ? Q.ncoarse : Q.nfine;
-                const CoopDesc &F = A.d[Q.df], &Cd = A.d[Q.dc];
-                const int pf = (F.parity0 + (k + 1) * F.substeps) & 1, pc = (Cd.parity0 + (k + 1) * Cd.substeps) & 1;
-                const CoopSide fine{F.L, strides + Q.df, pf}, coarse{Cd.L, strides + Q.dc, pc};
-#pragma unroll 1
-                for (int i; (i = claim.mine - claim.base) < rr.n; claim.claim())
+                if (RES && diff && ph == 0) block_sums(acc->x, acc->y, s_sums);
+                const bool end = k + 1 == A.nsteps && ph + 1 == A.nphase && A.nwave == 0;
+                if (RES && diff && ph == 0)
                 {
-                    const int r = (rr.lo + i) * 8 + lane / 4;
-                    const bool valid = r < nrows;
-                    const float *m = sm + (size_t)(rr.line + i * (kind == 0 ? kCoopCoarseLines : kCoopFineLines)) * 32;
-                    const bool slow = __any_sync(0xffffffffu, __float_as_int(m[(kind == 0 ? 2 : 11) * 32 + lane]) != 0);
-                    if (kind == 0)
+                    double *red = A.d[0].C.red + (size_t)((uint32_t)(A.slot0 + k) % (uint32_t)A.ring) * 4;
+                    if (!end)
                     {
-                        const CoarseRowDev &row = Q.coarse[valid ? r : 0];
-                        if (!slow) coop_coarse(fine, coarse, F.C, m, valid);
-                        else if (pf) coarse_row<1>(F.L, Cd.L, F.C, row, lane & 3, valid, pc);
-                        else coarse_row<0>(F.L, Cd.L, F.C, row, lane & 3, valid, pc);
+                        target += gridDim.x;
+                        if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next, s_sums, red)) return false;
+                        continue;
                     }
-                    else
-                    {
-                        const FineRowDev &row = Q.fine[valid ? r : 0];
-                        if (!slow) coop_fine(fine, coarse, F.C, m, valid);
-                        else if (pc) fine_child<1>(F.L, Cd.L, F.C, row, lane & 3, valid, pf);
-                        else fine_child<0>(F.L, Cd.L, F.C, row, lane & 3, valid, pf);
-                    }
+                    __syncthreads();
+                    if (warp == 1) add_block_sums(s_sums, red);
                 }
-                claim.base += rr.n;
+                if (end) break;
+                target += gridDim.x;
+                if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next)) return false;
             }
-            if (k + 1 == A.nsteps && w + 1 == A.nwave) break;
-            target += gridDim.x;
-            if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next)) return coop_gave_up(A);
+#pragma unroll 1
+            for (int w = 0; w < A.nwave; w++)
+            {
+                CoopClaim claim(&s_next);
+#pragma unroll 1
+                for (int p = 0; p < A.np; p++)
+                {
+                    const CoopPair &Q = A.p[p];
+                    const int kind = Q.l1 - 1 == w ? 0 : Q.l1 == w ? 1 : -1; // coarse rows / fine rows
+                    if (kind < 0) continue;
+                    const CoopRange rr = rows[p * 2 + kind];
+                    const int nrows = kind == 0 ? Q.ncoarse : Q.nfine;
+                    const CoopDesc &F = A.d[Q.df], &Cd = A.d[Q.dc];
+                    const int pf = (F.parity0 + (k + 1) * F.substeps) & 1, pc = (Cd.parity0 + (k + 1) * Cd.substeps) & 1;
+                    const CoopSide fine{F.L, strides + Q.df, pf}, coarse{Cd.L, strides + Q.dc, pc};
+#pragma unroll 1
+                    for (int i; (i = claim.mine - claim.base) < rr.n; claim.claim())
+                    {
+                        const int r = (rr.lo + i) * 8 + lane / 4;
+                        const bool valid = r < nrows;
+                        const float *m = sm + (size_t)(rr.line + i * (kind == 0 ? kCoopCoarseLines : kCoopFineLines)) * 32;
+                        const bool slow = __any_sync(0xffffffffu, __float_as_int(m[(kind == 0 ? 2 : 11) * 32 + lane]) != 0);
+                        if (kind == 0)
+                        {
+                            const CoarseRowDev &row = Q.coarse[valid ? r : 0];
+                            if (!slow) coop_coarse(fine, coarse, F.C, m, valid);
+                            else if (pf) coarse_row<1>(F.L, Cd.L, F.C, row, lane & 3, valid, pc);
+                            else coarse_row<0>(F.L, Cd.L, F.C, row, lane & 3, valid, pc);
+                        }
+                        else
+                        {
+                            const FineRowDev &row = Q.fine[valid ? r : 0];
+                            if (!slow) coop_fine(fine, coarse, F.C, m, valid);
+                            else if (pc) fine_child<1>(F.L, Cd.L, F.C, row, lane & 3, valid, pf);
+                            else fine_child<0>(F.L, Cd.L, F.C, row, lane & 3, valid, pf);
+                        }
+                    }
+                    claim.base += rr.n;
+                }
+                if (k + 1 == A.nsteps && w + 1 == A.nwave) break;
+                target += gridDim.x;
+                if (!grid_barrier(A.bar, target, A.polls, nullptr, nullptr, &s_next)) return false;
+            }
         }
-    }
-    if (RES)
+        return true;
+    };
+    const bool ok = steps();
+    coop_leave(A, ok);
+    if (RES && ok)
     {
         __syncthreads(); // the last stage has no barrier: other warps' |u| are still being stored
+        if (warp == 0) coop_place_cells(A, rng);
+        __syncthreads();
         coop_cells<true, RES>(A, rng, sm);
     }
 }

@@ -301,6 +301,8 @@ struct mgpu_ctx
     std::vector<std::unique_ptr<PhasePlan>> level_plans; // single-level tables (mgpu_step_level)
     int sm_count = 1;
     int stream_sms = 1; // of these, what kernels on `stream` can use
+    int64_t l2 = 0;          // bytes of the device's L2 cache
+    int64_t populations = 0; // bytes of the levels' dense population planes
     double autotune_us[3] = {0.0, 0.0, 0.0}; // plain_path -1: microseconds per coarse step of paths 0, 1, 2
     int64_t coarse_done = 0;     // coarse steps executed since creation
     int64_t ref_t = 0;           // reference lb->t
@@ -1046,7 +1048,6 @@ void run_coop(CoopPlan &P, int n, int every, bool skip_first, unsigned int *bar,
                 A.d[d].parity0 = (int)(l.steps & 1);
                 A.d[d++].direct0 = l.steps == 0 ? 1 : 0;
             }
-        CK(cudaMemsetAsync(bar, 0, sizeof(unsigned int), st));
         void *args[] = {&A};
         CK(cudaLaunchCooperativeKernel(P.kernel[every > 0], dim3((unsigned)P.grid), dim3((unsigned)P.threads[every > 0]), args, P.smem[every > 0], st));
         launches++;
@@ -1066,21 +1067,47 @@ bool is_capturing(cudaStream_t s)
     return cs != cudaStreamCaptureStatusNone;
 }
 
-// A transport context steps by cooperative launches unless the caller chose a
-// plain-cell kernel (plain_path), the launch engine, or said that other contexts
-// share the GPU.  Its blocks are one per SM of the device (the shares of the cells
-// are made for them) and must be resident together: a stream of fewer SMs takes
-// the launches.
-bool coop_ok(mgpu_ctx *ctx, bool residual)
+// How a call of n coarse steps of a transport context is stepped: in cooperative
+// launches unless the caller chose a plain-cell kernel (plain_path), the launch
+// engine, or said that other contexts share the GPU.  The blocks of such a launch are
+// one per SM of the device (the shares of the cells are made for them) and must be
+// resident together: a stream of fewer SMs takes the launches.
+enum class Route
+{
+    kCoop,
+    kLaunches, // per phase; pairs of steps from a graph
+    kSteps,    // launches per phase, step by step: the graph is bound to the parity that
+               // it was captured at, and calls of one step change that
+};
+enum class Entry
+{
+    kRun,     // mgpu_run: residuals
+    kAdvance, // mgpu_advance: residuals
+    kGraph,   // mgpu_advance_graph
+};
+Route coop_route(mgpu_ctx *ctx, Entry entry, int n)
 {
     if (ctx->adsorption || ctx->engine != MGPU_ENGINE_PERSISTENT || ctx->prm.plain_path >= 0 || ctx->prm.concurrent)
-        return false;
+        return Route::kLaunches;
     if (!ctx->coop)
     {
-        if (is_capturing(ctx->stream)) return false; // nothing is allocated during a capture
+        if (is_capturing(ctx->stream)) return Route::kLaunches; // nothing is allocated during a capture
         ctx->coop = build_coop({ctx});
     }
-    return ctx->coop->grid <= ctx->stream_sms && (residual ? ctx->coop->ok_residual : ctx->coop->ok);
+    const bool residual = entry != Entry::kGraph;
+    if (ctx->coop->grid > ctx->stream_sms || !(residual ? ctx->coop->ok_residual : ctx->coop->ok)) return Route::kLaunches;
+    // A launch begins with the fill of its blocks' shared memory and, with residuals,
+    // ends with the stored |u| on its way back.  Where the populations are beyond the L2
+    // that takes more than one or two steps gain (us per call, cooperative / launches, 2048^2,
+    // one level: 1 step 82 / 65, 2 steps 128 / 117, 4 steps 216 / 226; two levels: 122 / 109,
+    // 208 / 201, 383 / 390), and two levels with residuals never gain (1 step 182 / 151, 8 steps
+    // 1047 / 1014, 100 steps 12400 / 12400).  A run of a single step costs more beyond a
+    // quarter of the L2 (1024^2 197 / 192, 1500^2 362 / 347; 700^2 125 / 127).
+    const bool large = ctx->populations > ctx->l2;
+    if (large && residual && ctx->lay.max_level > 1) return Route::kLaunches;
+    if ((large && n <= 2) || (entry == Entry::kRun && n == 1 && ctx->populations > ctx->l2 / 4))
+        return is_capturing(ctx->stream) ? Route::kCoop : Route::kSteps; // (the launches' graph is not recorded)
+    return Route::kCoop;
 }
 
 // Steps recorded by a caller's stream capture hold the parity of each level and
@@ -1137,7 +1164,8 @@ void run_batch_with_residuals(mgpu_ctx *ctx, int n)
         }
         return;
     }
-    if (n > 0 && coop_ok(ctx, true))
+    const Route route = n > 0 ? coop_route(ctx, Entry::kRun, n) : Route::kLaunches;
+    if (route == Route::kCoop)
         run_coop(*ctx->coop, n, 1, true, ctx->grid_bar.p, ctx->stream, ctx->launches);
     else
     {
@@ -1145,7 +1173,7 @@ void run_batch_with_residuals(mgpu_ctx *ctx, int n)
         {
             int64_t k = ctx->coarse_done + 1; // this step
             bool diff = i > 0;                // residual of step k-1 (the previous batch closed its own last one)
-            if (diff && graphs && n - i >= 2 && !fresh_state(ctx))
+            if (diff && graphs && route != Route::kSteps && n - i >= 2 && !fresh_state(ctx))
             {
                 run_pair_graph(ctx, true, (int)((k - 1) % kRing));
                 i += 2;
@@ -1790,6 +1818,9 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
 
     CK(cudaGetDevice(&ctx->device));
     CK(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device));
+    int l2 = 0;
+    CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device));
+    ctx->l2 = l2;
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     ctx->own_stream = true;
     ctx->stream_sms = sms_of_stream(ctx->stream, ctx->sm_count);
@@ -1803,6 +1834,7 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
         const LevelLayout &ll = ctx->lay.levels[l];
         LevelDev &d = ctx->lv[l];
         d.f.alloc((size_t)ll.plane * 9, acct);
+        ctx->populations += (int64_t)d.f.n * (int64_t)sizeof(float);
         d.f.zero(s);
         d.omega.upload(ll.omega, acct, s);
         if (p->plain_path != 0 && !ctx->adsorption && ll.n_tiles_interior > 0)
@@ -1873,7 +1905,8 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
     ctx->red.zero(s);
     ctx->errword.alloc(1, acct);
     ctx->errword.zero(s);
-    ctx->grid_bar.alloc(1, acct);
+    ctx->grid_bar.alloc(2, acct);
+    ctx->grid_bar.zero(s);
     for (auto &it : ctx->lay.interfaces)
     {
         ctx->itf.emplace_back();
@@ -2065,7 +2098,10 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
         };
         // with a residual every step, pairs of steps replay a CUDA graph (not for
         // coupled runs, whose phase switch is host-side, nor from the initial state)
-        auto pairs_ok = [&](int i) { return K == 1 && !ctx->coupled && n_steps - i >= 2 && !fresh_state(ctx); };
+        const Route route = n_steps > 0 ? coop_route(ctx, Entry::kAdvance, n_steps) : Route::kLaunches;
+        auto pairs_ok = [&](int i) {
+            return K == 1 && !ctx->coupled && route != Route::kSteps && n_steps - i >= 2 && !fresh_state(ctx);
+        };
         for (int i = 0; i < n_steps; i++)
         {
             int64_t k = ctx->coarse_done + 1;
@@ -2108,7 +2144,7 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
                 if ((int)pending.size() >= kRing / 2) flush();
                 continue;
             }
-            if (coop_ok(ctx, true))
+            if (route == Route::kCoop)
             {
                 // the rest of the call (as many steps as the pending slots hold) in one launch
                 const int m = std::min(n_steps - i, kRing / 2 - (int)pending.size());
@@ -2162,7 +2198,14 @@ int mgpu_advance_graph(mgpu_ctx *ctx, int n_steps)
             ctx->ref_t += n_steps;
             return MGPU_OK;
         }
-        if (coop_ok(ctx, false))
+        const Route route = coop_route(ctx, Entry::kGraph, n_steps);
+        if (route == Route::kSteps)
+        {
+            for (int i = 0; i < n_steps; i++) coarse_step(ctx, false, false, 0);
+            ctx->ref_t += n_steps;
+            return MGPU_OK;
+        }
+        if (route == Route::kCoop)
         {
             check_replayable(ctx, n_steps);
             run_coop(*ctx->coop, n_steps, 0, false, ctx->grid_bar.p, ctx->stream, ctx->launches);
@@ -2701,6 +2744,7 @@ struct mgpu_batch
     std::vector<std::unique_ptr<CoopPlan>> coop;
     std::map<std::string, std::unique_ptr<PersistPlan>> pplans;
     DevBuf<unsigned int> sync; // claim and stage counters of the persistent launch
+    DevBuf<unsigned int> grid_bar; // grid-barrier arrivals of the cooperative launches
     int64_t bytes = 0;
     int sm_count = 1, stream_sms = 1;
 };
@@ -2725,33 +2769,44 @@ void batch_leave(mgpu_batch *b)
         if (c->stream != b->stream) CK(cudaStreamWaitEvent(c->stream, b->ev_done, 0));
 }
 
-// Groups of the batch's images for the cooperative engine, in order: as many
-// together as their state fits twice the L2 (dense planes, of which a step touches
-// the cells' sectors) and the kernel's tables.  us per coarse step of a batch with
-// groups of 1x / 2x / 4x the L2: four 1024^2 images of two levels 137 / 130 / 142
-// (the launch engine: 141), of one level 48 / 44 / 62 (58), six of mixed sizes
-// 84 / 58 / 58 (62).  Images beyond that size keep the launch engine, whose
-// images overlap (two 2048^2 images of two levels: 197, launches 186).
-bool batch_coop(mgpu_batch *b)
+// Groups of the batch's images for the cooperative engine, in order: as many together
+// as their populations (dense planes, of which a step touches the cells' sectors) fit
+// three quarters of the L2 and the kernel's tables.  us per coarse step of a batch in
+// groups of up to 0.4x / 0.75x / 1x / 1.5x the L2, and by the launch engine: four 1024^2
+// images of one level 46.7 / 41.9 / 42.8 / 61.1, 58.5, of two 139.4 / 133.8 / 133.8 / 133.8, 138.8;
+// sixteen of 512^2 52.0 / 45.5 / 69.1 / 69.1, 98.3; six of mixed sizes 77.5 / 57.2 / 57.2 / 57.2, 60.6.
+// Two 2048^2 images, each in launches of its own: 89.6 (one level), 176 (two); the
+// launch engine, whose images overlap, 114 and 188.  Beside such an image small ones
+// are groups that nothing overlaps (128^2, 512^2, 2048^2 and 256^2: 142, launches 105):
+// these batches keep the launch engine.
+// Few steps of few images stay with the launch engine (up to 2 of one level, else 6): a
+// group's launch costs 25 to 35 us beside its steps, and the launch engine's graph holds
+// two steps (four 1024^2 images, 2 / 4 / 10 steps: one level 129 / 211 / 460, launches 123 / 233 /
+// 582; two levels 339 / 607 / 1404, 281 / 560 / 1394).  More levels make more launches per step (eight 512^2 images of two levels, 2
+// steps: 235, launches 238), and an odd number of steps leaves the graph's parity.
+bool batch_coop(mgpu_batch *b, int n_steps)
 {
     if (b->coop.empty())
     {
         if (is_capturing(b->stream)) return false; // nothing is allocated during a capture
-        int l2 = 0;
-        CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, b->ctxs[0]->device));
-        const int64_t most = 2 * (int64_t)l2;
-        for (auto *c : b->ctxs)
-            if (c->bytes > most) return false;
         std::vector<int64_t> bytes;
-        for (auto *c : b->ctxs) bytes.push_back(c->bytes);
-        b->coop = coop_groups<CoopPlan>(bytes, most, [&](size_t first, size_t count) {
+        for (auto *c : b->ctxs) bytes.push_back(c->populations);
+        b->coop = coop_groups<CoopPlan>(bytes, b->ctxs[0]->l2 / 4 * 3, [&](size_t first, size_t count) {
             const auto at = b->ctxs.begin() + (std::ptrdiff_t)first;
             return build_coop(std::vector<mgpu_ctx *>(at, at + (std::ptrdiff_t)count));
         });
     }
     for (auto &g : b->coop)
         if (!g->ok || g->grid > b->stream_sms) return false;
-    return true;
+    size_t levels = 0, large = 0;
+    for (auto *c : b->ctxs)
+    {
+        levels += c->lv.size();
+        large += c->populations > c->l2 ? 1 : 0;
+    }
+    if (large > 0 && large < b->ctxs.size()) return false;
+    const bool few = n_steps < (levels == b->ctxs.size() ? 4 : 8) && (n_steps % 2 == 0 || (n_steps == 1 && b->coop.size() > 1));
+    return !(few && levels <= 12);
 }
 
 // the persistent plan of the batch's current state for n coarse steps
@@ -2867,6 +2922,8 @@ int mgpu_batch_create(mgpu_ctx *const *ctxs, int n, mgpu_batch **out)
         // stage counters of two coarse steps: at most 2^(L-1) phases and L waves
         // per image and step (L <= 4)
         b->sync.alloc(1 + b->ctxs.size() * 2 * (8 + 4), b->bytes);
+        b->grid_bar.alloc(2, b->bytes);
+        b->grid_bar.zero(b->stream);
         *out = b.release();
         return MGPU_OK;
     });
@@ -2877,11 +2934,11 @@ int mgpu_batch_advance(mgpu_batch *b, int n_steps)
     return guarded(nullptr, [&]() {
         if (!b || n_steps < 0) throw std::invalid_argument("bad argument");
         batch_enter(b);
-        if (!b->engine_set && batch_coop(b))
+        if (!b->engine_set && batch_coop(b, n_steps))
         {
             for (auto &g : b->coop)
             {
-                run_coop(*g, n_steps, 0, false, b->sync.p, b->stream, b->launches);
+                run_coop(*g, n_steps, 0, false, b->grid_bar.p, b->stream, b->launches);
                 for (auto *c : g->ctxs) c->ref_t += n_steps;
             }
             batch_leave(b);

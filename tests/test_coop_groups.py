@@ -36,13 +36,14 @@ int main()
     show(make({1, 1, 1, 1, 1, 1, 1, 1, 1}, 100, 0));
     show(make({1000, 1, 1000, 2}, 5000, 0));
     show(make({}, 1, 0));
-    Groups held; // as the batch holds them
-    for (int k = 1; k <= 6; k++)
-    {
-        bool thrown = false;
-        try { held = make({4, 4, 4, 4, 4}, 8, k); } catch (const std::runtime_error &) { thrown = true; }
-        std::printf("%d:%d:%zu ", k, (int)thrown, held.size());
-    }
+    show(make({5, 5, 5, 5, 5, 5}, 24, 0)); // 4 + 2 -> 3 + 3
+    show(make({9, 1, 1, 1, 1, 1, 1}, 12, 0));
+    show(make({2, 3, 4, 5, 6, 7}, 14, 0));
+    Groups held; // as the batch holds them: none until a build of every one succeeds
+    int thrown = 0;
+    for (int k = 1; held.empty() && k < 1000; k++)
+        try { held = make({4, 4, 4, 4, 4}, 8, k); } catch (const std::runtime_error &) { thrown++; }
+    std::printf("%s %zu", thrown >= 5 ? "thrown" : "", held.size());
     std::printf("\n");
 }
 """
@@ -57,9 +58,11 @@ def test_groups(tmp_path):
     assert [l.strip() for l in lines] == [
         "0+3",
         "0+2 2+1 3+1 4+2",
-        "0+4 4+4 8+1",
+        "0+3 3+3 6+3",
         "0+1! 1+1 2+1! 3+1",
         "",
-        # five images in three groups take five builds; none is held before the sixth try
-        "1:1:0 2:1:0 3:1:0 4:1:0 5:1:0 6:0:3",
+        "0+3 3+3",
+        "0+3 3+4",
+        "0+4 4+2",
+        "thrown 3",
     ]
