@@ -411,6 +411,12 @@ int conv(const float *x, const uint16_t *w, const float *b, float *y, const floa
     }
 }
 
+// two blocks per SM share a channel group's pixel tiles
+int64_t wgrad_split(int64_t groups, int64_t tiles, int sms)
+{
+    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(tiles, 65535), 2 * sms / groups));
+}
+
 template <typename T>
 int launch_wgrad(const float *x, const float *dy, float *dw, float *db, int n, int cin, int cout, int h, int wd,
                  cudaStream_t st)
@@ -421,11 +427,50 @@ int launch_wgrad(const float *x, const float *dy, float *dw, float *db, int n, i
     if (e != cudaSuccess) return -(int)e;
     const int64_t groups = (int64_t)((cout + T::CO - 1) / T::CO) * ((cin + T::LCI - 1) / T::LCI);
     const int64_t tiles = (int64_t)((wd + T::TW - 1) / T::TW) * ((h + T::TH - 1) / T::TH) * n;
-    // two blocks per SM share a channel group's pixel tiles
-    const int64_t split = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(tiles, 65535), 2 * sm_count() / groups));
-    kernel<<<dim3((unsigned)groups, (unsigned)split), cnn_fma::kThreads, T::kSmem, st>>>(x, dy, dw, db, n, cin, cout, h, wd);
+    kernel<<<dim3((unsigned)groups, (unsigned)wgrad_split(groups, tiles, sm_count())), cnn_fma::kThreads, T::kSmem, st>>>(x, dy, dw, db, n, cin, cout, h, wd);
     return done();
 }
+
+// The weight gradient's tile for a layer by a model of its time, in packed FMAs of a
+// thread: rounds of blocks over the SMs, each block's tiles one after the other (FMAs of
+// its thread, 41 per copy of inputs and 31 of gradients that a thread stages; two blocks
+// on an SM halve its rate; no tile below 182), and the sums at the end.  The numbers
+// are fitted to every tile's times on 634 layers.
+struct WgradChoice
+{
+    typedef int (*Launch)(const float *, const float *, float *, float *, int, int, int, int, int, cudaStream_t);
+    int n, cin, cout, h, wd, sms;
+    double cost = 0.0, limit = 0.0;
+    Launch launch = nullptr;
+    template <typename T> double time() const
+    {
+        const int64_t groups = (int64_t)((cout + T::CO - 1) / T::CO) * ((cin + T::LCI - 1) / T::LCI);
+        const int64_t tiles = (int64_t)((wd + T::TW - 1) / T::TW) * ((h + T::TH - 1) / T::TH) * n;
+        const int64_t split = wgrad_split(groups, tiles, sms), blocks = groups * split;
+        const double share = blocks <= sms ? 1.0 : 2.0, rounds = (double)std::max<int64_t>(1, (blocks + 2 * sms - 1) / (2 * sms));
+        const double fma = 18.0 * T::TW * T::TH / T::SPLIT;
+        const double x = T::LCI * (T::TH + 2) * (wd % 4 == 0 ? T::TW / 4 + 2 : T::TW + 2) / (double)cnn_fma::kThreads;
+        const double y = T::CO * T::TW * T::TH / (double)cnn_fma::kThreads;
+        const double tile = std::max(182.0, share * (fma + 41.0 * x + 31.0 * y));
+        return rounds * (double)((tiles + split - 1) / split) * tile + 35.0 + 3.1 * T::CO * T::RUN / cnn_fma::kThreads;
+    }
+    template <typename T> void start()
+    {
+        cost = time<T>();
+        // (where every block has one tile and all run at once, the model is closer)
+        const int64_t groups = (int64_t)((cout + T::CO - 1) / T::CO) * ((cin + T::LCI - 1) / T::LCI);
+        const int64_t tiles = (int64_t)((wd + T::TW - 1) / T::TW) * ((h + T::TH - 1) / T::TH) * n;
+        limit = (groups * tiles <= 2 * sms ? 0.8 : 0.575) * cost;
+        launch = launch_wgrad<T>;
+    }
+    template <typename T> void other()
+    {
+        const double c = time<T>();
+        if (c >= limit || c >= cost) return;
+        cost = c;
+        launch = launch_wgrad<T>;
+    }
+};
 } // namespace
 
 extern "C" {
@@ -525,15 +570,30 @@ int cnn_conv3x3_backward_weight(const float *x, const float *dy, float *dw, floa
 {
     if (n <= 0 || cin <= 0 || cout <= 0 || h <= 0 || wd <= 0) return -1;
     const cudaStream_t st = (cudaStream_t)stream;
-    // 16 x 8 pixel tiles, 8 x 8 where the image is no wider; with few output
-    // (input) channels the warps (lanes) share the pixels instead of channels
     using namespace cnn_fma;
+    WgradChoice pick{n, cin, cout, h, wd, sm_count()};
+    // 16 x 8 pixel tiles and 32 x 32 channels, 8 x 8 where the image is no wider; with few
+    // output (input) channels the warps (lanes) share the pixels instead of channels
     if (cout <= 8)
-        return wd > 8 ? launch_wgrad<WgradTile<16, 8, 1, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st)
-                      : launch_wgrad<WgradTile<8, 8, 1, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st);
-    if (cin <= 4) return launch_wgrad<WgradTile<16, 8, 8, 4>>(x, dy, dw, db, n, cin, cout, h, wd, st);
-    return wd > 8 ? launch_wgrad<WgradTile<16, 8, 8, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st)
-                  : launch_wgrad<WgradTile<8, 8, 8, 32>>(x, dy, dw, db, n, cin, cout, h, wd, st);
+    {
+        if (wd > 8) pick.start<WgradTile<16, 8, 1, 32>>();
+        else pick.start<WgradTile<8, 8, 1, 32>>();
+    }
+    else if (cin <= 4) pick.start<WgradTile<16, 8, 8, 4>>();
+    else if (wd > 8) pick.start<WgradTile<16, 8, 8, 32>>();
+    else pick.start<WgradTile<8, 8, 8, 32>>();
+    // Smaller tiles where few blocks, or channels that are not there, leave those waiting: 4
+    // or 8 output channels x 8 input channels, 16 x 16 on 16 x 8 or 8 x 8 pixels.  Only where
+    // the model sees a good deal to gain: of 634 layers (1 to 8 images, 1 to 256 channels, 4 to
+    // 140 pixels) none was more than 1.5 % slower for it, and the choice is 4 % from the best of 21
+    // tiles on the average (30 % without).  us, with the tile above / now / with tiles of 16^2 pixels and
+    // channels before these kernels: 11 -> 34 channels at 57^2 (5 images) 33 / 19 / 22, 34 -> 13 at 102 x 25
+    // (6) 33 / 19 / 23, 2 -> 5 at 129^2 (8) 50 / 17 / 40, 251 -> 12 at 20^2 (6) 22 / 14.5 / 28.
+    pick.other<WgradTile<16, 8, 1, 8>>();
+    pick.other<WgradTile<16, 8, 2, 8>>();
+    pick.other<WgradTile<16, 8, 4, 16>>();
+    pick.other<WgradTile<8, 8, 4, 16>>();
+    return pick.launch(x, dy, dw, db, n, cin, cout, h, wd, st);
 }
 
 int cnn_relu_backward(float *dy, const float *y, int64_t count, void *stream)
