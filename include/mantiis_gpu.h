@@ -63,7 +63,9 @@ typedef struct mgpu_params
                               (the state is put back; results are bit-identical on every path) */
     int concurrent;        /* 1: other contexts step on this GPU at the same time (several host threads or
                               streams); the 8x4 plain kernel then leaves room on every SM for their kernels
-                              (a batch does this by itself).  0 (default): this context has the GPU */
+                              (a batch does this by itself) and no cooperative launches are made.  0 (default):
+                              a call that finds steps of other contexts or batches in flight shares the GPU
+                              with them, else it has the GPU (mgpu_set_engine) */
 } mgpu_params;
 
 /* Static description of a built context. */
@@ -264,7 +266,10 @@ int mgpu_batch_set_engine(mgpu_batch *b, int engine, int group);
  * seconds, then MGPU_E_DEVICE); engine 0 launches the passes or phases of every
  * step (pairs of steps replayed from a CUDA graph).  Both give bit-identical
  * states.  A transport context uses engine 0 all the same where plain_path names a
- * kernel of it or `concurrent` says that other contexts share the GPU. */
+ * kernel of it, where `concurrent` says that other contexts share the GPU, for one or two
+ * steps of images beyond the L2 cache, on a stream of fewer SMs than the device has, and
+ * while steps of other contexts of the process are in flight if the image is one of
+ * those that step faster side by side than in turns (about 150^2 to 700^2). */
 int mgpu_set_engine(mgpu_ctx *ctx, int engine);
 /* How often a block polls at a grid barrier of this context's cooperative launches
  * (in a batch: of the group whose first image the context is) before it gives up:

@@ -216,6 +216,98 @@ struct SideLanes
     }
 };
 
+// Transport steps of a context or a batch that are being enqueued or may still run.
+// Cooperative launches hold every SM, launches per phase share them; which of the two
+// a call should take depends on whether others step on the device at the same time
+// (other host threads, other streams), and this is how a call sees it: every step call
+// opens and closes on its activity, and looks at those of the others.  Only the way of
+// stepping follows from it, never a state.
+class StepActivity
+{
+  public:
+    explicit StepActivity(int dev) : device(dev)
+    {
+        CK(cudaEventCreateWithFlags(&queued, cudaEventDisableTiming));
+        std::lock_guard<std::mutex> hold(lock());
+        all().push_back(this);
+    }
+    ~StepActivity()
+    {
+        {
+            std::lock_guard<std::mutex> hold(lock());
+            all().erase(std::find(all().begin(), all().end(), this));
+        }
+        cudaEventDestroy(queued);
+    }
+    StepActivity(const StepActivity &) = delete;
+    StepActivity &operator=(const StepActivity &) = delete;
+
+    // One call; `own`: activities that are no others to it (a batch's contexts).  Nothing
+    // is looked at or noted in a stream capture.
+    class Call
+    {
+      public:
+        bool shared = false; // others step now
+        Call(StepActivity &a, cudaStream_t st, const std::vector<StepActivity *> &own = {}) : self(a), stream(st)
+        {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            CK(cudaStreamIsCapturing(st, &cs));
+            counted = cs == cudaStreamCaptureStatusNone;
+            if (!counted) return;
+            // (an event is asked for here: another thread's capture does not mind)
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            {
+                std::lock_guard<std::mutex> hold(lock());
+                for (StepActivity *o : all())
+                {
+                    if (shared) break;
+                    if (o == &self || o->device != self.device || std::find(own.begin(), own.end(), o) != own.end()) continue;
+                    if (o->noted && cudaEventQuery(o->queued) != cudaErrorNotReady) o->noted = false;
+                    shared = o->calls > 0 || o->noted;
+                }
+                self.calls++;
+            }
+            cudaGetLastError();
+            cudaThreadExchangeStreamCaptureMode(&mode);
+        }
+        // the call returns with its work still queued on the stream
+        void leaves_work()
+        {
+            if (!counted) return;
+            std::lock_guard<std::mutex> hold(lock());
+            self.noted = cudaEventRecord(self.queued, stream) == cudaSuccess;
+        }
+        ~Call()
+        {
+            if (!counted) return;
+            std::lock_guard<std::mutex> hold(lock());
+            self.calls--;
+        }
+
+      private:
+        StepActivity &self;
+        cudaStream_t stream;
+        bool counted = false;
+    };
+
+  private:
+    static std::mutex &lock()
+    {
+        static std::mutex *m = new std::mutex(); // outlives every context
+        return *m;
+    }
+    static std::vector<StepActivity *> &all()
+    {
+        static auto *v = new std::vector<StepActivity *>();
+        return *v;
+    }
+    int device;
+    cudaEvent_t queued = nullptr;
+    bool noted = false; // `queued` was recorded and not yet seen done
+    int calls = 0;
+};
+
 // Captures the work enqueued on `st` between construction and take() into a
 // graph; if an exception leaves the scope first, the capture is ended and its
 // partial graph dropped, so the stream is usable again.
@@ -301,6 +393,7 @@ struct mgpu_ctx
     std::vector<std::unique_ptr<PhasePlan>> level_plans; // single-level tables (mgpu_step_level)
     int sm_count = 1;
     int stream_sms = 1; // of these, what kernels on `stream` can use
+    std::unique_ptr<StepActivity> activity; // of transport contexts
     int64_t l2 = 0;          // bytes of the device's L2 cache
     int64_t populations = 0; // bytes of the levels' dense population planes
     double autotune_us[3] = {0.0, 0.0, 0.0}; // plain_path -1: microseconds per coarse step of paths 0, 1, 2
@@ -1024,15 +1117,21 @@ std::unique_ptr<CoopPlan> build_coop(const std::vector<mgpu_ctx *> &ctxs)
 
 // n coarse steps of the plan's images in one launch on `st`.  every > 0 (one
 // image): residuals as dev::CoopLaunch describes, into zeroed slots.
-void run_coop(CoopPlan &P, int n, int every, bool skip_first, unsigned int *bar, cudaStream_t st, int64_t &launches)
+void run_coop(CoopPlan &P, int n, int every, bool skip_first, unsigned int *bar, cudaStream_t st, int64_t &launches,
+              bool shared)
 {
     dev::CoopLaunch &A = P.L;
     // a launch holds every SM: other streams' kernels get their turn between
-    // launches (the fill of shared memory at its start takes about 10 us)
-    constexpr int kMaxSteps = 500;
+    // launches (the fill of shared memory at its start takes about 10 us).  Turns are short
+    // where other contexts step now: 400 steps of a 128^2 image beside a two-level
+    // 1024^2 image that steps 500 at a time took 19 ms, with launches of 32 steps 3.2 (launches
+    // per phase of both: 4.6)
+    int64_t cells = 0;
+    for (auto *c : P.ctxs) cells += c->grid.n_cells;
+    const int most = shared && cells > 130 * P.grid ? 32 : 500;
     for (int done = 0; done < n;)
     {
-        A.nsteps = std::min(kMaxSteps, n - done);
+        A.nsteps = std::min(most, n - done);
         A.every = every;
         // (the state before the first step of all has no stored |u|)
         A.skip_first = (skip_first && done == 0) || P.ctxs[0]->coarse_done == 0 ? 1 : 0;
@@ -1085,7 +1184,20 @@ enum class Entry
     kAdvance, // mgpu_advance: residuals
     kGraph,   // mgpu_advance_graph
 };
-Route coop_route(mgpu_ctx *ctx, Entry entry, int n)
+// Whether images of so many cells and levels step faster by cooperative launches, one
+// after the other, than by launches per phase side by side, where others step at the
+// same time.  Four contexts on four host threads, us per step of all, cooperative /
+// launches (mgpu_advance_graph; mgpu_run): one level 128^2 (9 k cells) 5.5 / 10.5; 6.7 / 17, 256^2
+// (38 k) 9.8 / 12.1; 23 / 18, 320^2 (60 k) 19 / 13; 23 / 20, 512^2 (156 k) 21 / 17; 30 / 35, 724^2 (313 k)
+// 30 / 29; 42 / 59, 1024^2 (629 k) 47 / 62; 64 / 119; two levels 256^2 66 / 33; 72 / 40, 512^2 (122 k) 82 / 52;
+// 85 / 68, 1024^2 (346 k) 137 / 154; 146 / 183; three levels 512^2 (161 k) 150 / 104; 168 / 126, 1024^2 (538 k)
+// 307 / 390; 337 / 441.
+bool coop_when_shared(int64_t cells, size_t levels, bool residual, int sms)
+{
+    return cells >= 2000 * sms || (levels == 1 && (cells <= 130 * sms || (residual && cells >= 700 * sms)));
+}
+
+Route coop_route(mgpu_ctx *ctx, Entry entry, int n, bool shared)
 {
     if (ctx->adsorption || ctx->engine != MGPU_ENGINE_PERSISTENT || ctx->prm.plain_path >= 0 || ctx->prm.concurrent)
         return Route::kLaunches;
@@ -1095,6 +1207,7 @@ Route coop_route(mgpu_ctx *ctx, Entry entry, int n)
         ctx->coop = build_coop({ctx});
     }
     const bool residual = entry != Entry::kGraph;
+    if (shared && !coop_when_shared(ctx->grid.n_cells, ctx->lv.size(), residual, ctx->sm_count)) return Route::kLaunches;
     if (ctx->coop->grid > ctx->stream_sms || !(residual ? ctx->coop->ok_residual : ctx->coop->ok)) return Route::kLaunches;
     // A launch begins with the fill of its blocks' shared memory and, with residuals,
     // ends with the stored |u| on its way back.  Where the populations are beyond the L2
@@ -1135,7 +1248,7 @@ bool fresh_state(const mgpu_ctx *ctx)
 // the residual of the last step comes from a read pass.  Pairs of steps run
 // from a CUDA graph (not for coupled runs, whose phase switch is host-side,
 // nor from the initial "direct" state).
-void run_batch_with_residuals(mgpu_ctx *ctx, int n)
+void run_batch_with_residuals(mgpu_ctx *ctx, int n, bool shared)
 {
     int64_t k0 = ctx->coarse_done;
     zero_slots(ctx, (int)((k0 + 1) % kRing), n);
@@ -1164,9 +1277,9 @@ void run_batch_with_residuals(mgpu_ctx *ctx, int n)
         }
         return;
     }
-    const Route route = n > 0 ? coop_route(ctx, Entry::kRun, n) : Route::kLaunches;
+    const Route route = n > 0 ? coop_route(ctx, Entry::kRun, n, shared) : Route::kLaunches;
     if (route == Route::kCoop)
-        run_coop(*ctx->coop, n, 1, true, ctx->grid_bar.p, ctx->stream, ctx->launches);
+        run_coop(*ctx->coop, n, 1, true, ctx->grid_bar.p, ctx->stream, ctx->launches, shared);
     else
     {
         for (int i = 0; i < n;)
@@ -1918,7 +2031,11 @@ static int create_impl(const PoreImage &img, const mgpu_params *p, mgpu_ctx **ou
         e.fine.upload(it.fine, acct, s);
     }
 
-    if (!ctx->adsorption) ctx->plan = build_plan({ctx.get()}, -1);
+    if (!ctx->adsorption)
+    {
+        ctx->plan = build_plan({ctx.get()}, -1);
+        ctx->activity.reset(new StepActivity(ctx->device));
+    }
 
     // initial state: rho = rho_init, u = 0, f = f_eq (include/coreLB.hpp:381-417)
     std::vector<double> rho(ctx->grid.n_cells, rho_init), zero(ctx->grid.n_cells, 0.0);
@@ -2028,9 +2145,12 @@ int mgpu_run(mgpu_ctx *ctx, int n_steps, int *steps_done)
             if (phase_a) batch = std::min(batch, 100 - ctx->coupled_a);
             checkpoint_save(ctx);
             int64_t k0 = ctx->coarse_done;
-            run_batch_with_residuals(ctx, batch);
+            std::unique_ptr<StepActivity::Call> call; // closed when its steps are done
+            if (ctx->activity) call.reset(new StepActivity::Call(*ctx->activity, ctx->stream));
+            run_batch_with_residuals(ctx, batch, call && call->shared);
             std::vector<double> slots((size_t)batch * 4);
             read_slots(ctx, (int)((k0 + 1) % kRing), batch, slots.data());
+            call.reset();
             int stop = -1;
             for (int i = 0; i < batch; i++)
             {
@@ -2098,7 +2218,10 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
         };
         // with a residual every step, pairs of steps replay a CUDA graph (not for
         // coupled runs, whose phase switch is host-side, nor from the initial state)
-        const Route route = n_steps > 0 ? coop_route(ctx, Entry::kAdvance, n_steps) : Route::kLaunches;
+        std::unique_ptr<StepActivity::Call> call;
+        if (ctx->activity) call.reset(new StepActivity::Call(*ctx->activity, ctx->stream));
+        const Route route =
+            n_steps > 0 ? coop_route(ctx, Entry::kAdvance, n_steps, call && call->shared) : Route::kLaunches;
         auto pairs_ok = [&](int i) {
             return K == 1 && !ctx->coupled && route != Route::kSteps && n_steps - i >= 2 && !fresh_state(ctx);
         };
@@ -2150,7 +2273,7 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
                 const int m = std::min(n_steps - i, kRing / 2 - (int)pending.size());
                 make_room(k - 1, m);
                 zero_slots(ctx, (int)((k - 1) % kRing), m);
-                run_coop(*ctx->coop, m, K, false, ctx->grid_bar.p, ctx->stream, ctx->launches);
+                run_coop(*ctx->coop, m, K, false, ctx->grid_bar.p, ctx->stream, ctx->launches, call && call->shared);
                 for (int64_t j = k; j < k + m; j++)
                     if (j >= 2 && (j - 1) % K == 0) pending.push_back(j - 1);
                 i += m - 1;
@@ -2182,6 +2305,7 @@ int mgpu_advance(mgpu_ctx *ctx, int n_steps)
             if ((int)pending.size() >= kRing / 2) flush();
         }
         flush();
+        if (call) call->leaves_work();
         ctx->ref_t += n_steps;
         return MGPU_OK;
     });
@@ -2198,17 +2322,21 @@ int mgpu_advance_graph(mgpu_ctx *ctx, int n_steps)
             ctx->ref_t += n_steps;
             return MGPU_OK;
         }
-        const Route route = coop_route(ctx, Entry::kGraph, n_steps);
+        std::unique_ptr<StepActivity::Call> call;
+        if (ctx->activity) call.reset(new StepActivity::Call(*ctx->activity, ctx->stream));
+        const Route route = coop_route(ctx, Entry::kGraph, n_steps, call && call->shared);
         if (route == Route::kSteps)
         {
             for (int i = 0; i < n_steps; i++) coarse_step(ctx, false, false, 0);
+            if (call) call->leaves_work();
             ctx->ref_t += n_steps;
             return MGPU_OK;
         }
         if (route == Route::kCoop)
         {
             check_replayable(ctx, n_steps);
-            run_coop(*ctx->coop, n_steps, 0, false, ctx->grid_bar.p, ctx->stream, ctx->launches);
+            run_coop(*ctx->coop, n_steps, 0, false, ctx->grid_bar.p, ctx->stream, ctx->launches, call && call->shared);
+            if (call) call->leaves_work();
             ctx->ref_t += n_steps;
             return MGPU_OK;
         }
@@ -2274,6 +2402,7 @@ int mgpu_advance_graph(mgpu_ctx *ctx, int n_steps)
             left -= 2;
         }
         if (left == 1) coarse_step(ctx, false, false, 0);
+        if (call) call->leaves_work();
         ctx->ref_t += n_steps;
         return MGPU_OK;
     });
@@ -2747,6 +2876,7 @@ struct mgpu_batch
     DevBuf<unsigned int> grid_bar; // grid-barrier arrivals of the cooperative launches
     int64_t bytes = 0;
     int sm_count = 1, stream_sms = 1;
+    std::unique_ptr<StepActivity> activity;
 };
 
 namespace
@@ -2919,6 +3049,7 @@ int mgpu_batch_create(mgpu_ctx *const *ctxs, int n, mgpu_batch **out)
         for (auto &e : b->ctx_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         b->sm_count = b->ctxs[0]->sm_count;
         b->stream_sms = sms_of_stream(b->stream, b->sm_count);
+        b->activity.reset(new StepActivity(dev));
         // stage counters of two coarse steps: at most 2^(L-1) phases and L waves
         // per image and step (L <= 4)
         b->sync.alloc(1 + b->ctxs.size() * 2 * (8 + 4), b->bytes);
@@ -2934,13 +3065,17 @@ int mgpu_batch_advance(mgpu_batch *b, int n_steps)
     return guarded(nullptr, [&]() {
         if (!b || n_steps < 0) throw std::invalid_argument("bad argument");
         batch_enter(b);
+        std::vector<StepActivity *> own;
+        for (auto *c : b->ctxs) own.push_back(c->activity.get());
+        StepActivity::Call call(*b->activity, b->stream, own);
         if (!b->engine_set && batch_coop(b, n_steps))
         {
             for (auto &g : b->coop)
             {
-                run_coop(*g, n_steps, 0, false, b->grid_bar.p, b->stream, b->launches);
+                run_coop(*g, n_steps, 0, false, b->grid_bar.p, b->stream, b->launches, call.shared);
                 for (auto *c : g->ctxs) c->ref_t += n_steps;
             }
+            call.leaves_work();
             batch_leave(b);
             return MGPU_OK;
         }
@@ -3025,6 +3160,7 @@ int mgpu_batch_advance(mgpu_batch *b, int n_steps)
             left -= 2;
         }
         if (left == 1) batch_step(b);
+        call.leaves_work();
         batch_leave(b);
         return MGPU_OK;
     });
