@@ -353,18 +353,16 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
         std::vector<char> is_buf((size_t)lv.plane, 0);
         for (size_t i = 0; i < L.buf_level.size(); i++)
             if (L.buf_level[i] == lv.level) is_buf[(size_t)L.buf_site[i]] = 1;
-        for (int kind = 0; kind < 2; kind++)
-        {
-            const size_t begin = lv.plain_xy.size();
-            for (int y = 0; y < lv.H; y++)
-                for (int x = 0; x < lv.W; x++)
-                {
-                    const size_t s = (size_t)y * lv.pitch + x;
-                    if (!(lv.omega[s] > 0.0f)) continue;
-                    if (is_buf[s] == kind) lv.plain_xy.push_back(x | y << 16);
-                }
-            lv.n_plain[kind] = (int64_t)(lv.plain_xy.size() - begin);
-        }
+        std::vector<int32_t> buffers;
+        for (int y = 0; y < lv.H; y++)
+            for (int x = 0; x < lv.W; x++)
+            {
+                const size_t s = (size_t)y * lv.pitch + x;
+                if (lv.omega[s] > 0.0f) (is_buf[s] ? buffers : lv.plain_xy).push_back(x | y << 16);
+            }
+        lv.n_plain[0] = (int64_t)lv.plain_xy.size();
+        lv.n_plain[1] = (int64_t)buffers.size();
+        lv.plain_xy.insert(lv.plain_xy.end(), buffers.begin(), buffers.end());
     }
 
     // 8x4 tiles holding a plain or light cell, row-major (one warp per tile in the
@@ -547,41 +545,5 @@ ImageLayout build_layout(const Grid &g, const LayoutParams &p)
     }
     L.tau_mean = nt ? ts / nt : 0.0;
     return L;
-}
-
-// Equal shares of a level's cells: lists sorted by site_order_key, cut where the
-// weight of all cells before the key reaches k / parts of the total.
-std::vector<std::vector<int32_t>> share_cuts(const std::vector<ShareList> &lists, int parts)
-{
-    double total = 0;
-    for (const ShareList &l : lists) total += l.weight * (double)l.n;
-    std::vector<std::vector<int32_t>> cuts(lists.size(), std::vector<int32_t>((size_t)parts + 1, 0));
-    std::vector<int32_t> at(lists.size(), 0);
-    double done = 0;
-    for (int k = 1; k <= parts; k++)
-    {
-        const double goal = total * k / parts;
-        while (k == parts || done < goal)
-        {
-            // the list whose next cell comes first
-            int best = -1;
-            uint32_t key = 0;
-            for (size_t l = 0; l < lists.size(); l++)
-            {
-                if (at[l] >= lists[l].n) continue;
-                const uint32_t kl = site_order_key(lists[l].xy[(size_t)at[l] * lists[l].stride]);
-                if (best < 0 || kl < key)
-                {
-                    best = (int)l;
-                    key = kl;
-                }
-            }
-            if (best < 0) break;
-            at[(size_t)best]++;
-            done += lists[(size_t)best].weight;
-        }
-        for (size_t l = 0; l < lists.size(); l++) cuts[l][(size_t)k] = at[l];
-    }
-    return cuts;
 }
 } // namespace mantiis

@@ -17,6 +17,8 @@
 #include <cstdint>
 #include <vector>
 
+#include "share_cuts.hpp"
+
 #include "../host/grid.hpp"
 
 namespace mantiis
@@ -157,24 +159,6 @@ struct ImageLayout
 };
 
 ImageLayout build_layout(const Grid &g, const LayoutParams &p);
-
-// Order of cells by place: row by row.  A contiguous share of such a list is a band
-// of the level, whatever the kind of cell, so the cells of one SM read each
-// other's sectors; long rows keep a warp's cells side by side (us per step of the
-// cooperative engine at 1024^2, single block / two levels, with the cells in
-// 32x32 tiles along a Z curve 13.6 / 39, 128x16 12.5 / 36, in rows 12.5 / 34).
-inline uint32_t site_order_key(int32_t xy) { return (uint32_t)xy; } // x | y << 16
-
-// one list of cells sorted by site_order_key: x | y << 16 of cell i at xy[i * stride]
-struct ShareList
-{
-    const int32_t *xy;
-    int32_t n;
-    int stride;
-    double weight; // work of a cell
-};
-// per list the parts + 1 cuts that give every part the same work and the same patch
-std::vector<std::vector<int32_t>> share_cuts(const std::vector<ShareList> &lists, int parts);
 
 // Interpolation weights of the reference's fine-buffer bicubic spline for one
 // parent (exposed for tests): nodes x[3], y[2] and the query points (qx, qy),
