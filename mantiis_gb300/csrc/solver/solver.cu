@@ -251,9 +251,12 @@ class StepActivity
         Call(StepActivity &a, cudaStream_t st, const std::vector<StepActivity *> &own = {}) : self(a), stream(st)
         {
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            CK(cudaStreamIsCapturing(st, &cs));
-            counted = cs == cudaStreamCaptureStatusNone;
-            if (!counted) return;
+            counted = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+            if (!counted)
+            {
+                cudaGetLastError();
+                return;
+            }
             // (an event is asked for here: another thread's capture does not mind)
             cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
             cudaThreadExchangeStreamCaptureMode(&mode);
