@@ -83,7 +83,8 @@ typedef struct mgpu_info
     double tau_mean;       /* mean tau_s over non-buffer cells (permeability viscosity) */
     int64_t device_bytes;  /* device memory held by the context */
     int64_t grid_undefined_cases; /* reference-undefined cases given a defined meaning */
-    int plain_path;        /* plain-cell path in use: 1 TMA pipeline, 0 direct 32x8, 2 direct 8x4 */
+    int plain_path;        /* plain-cell path of the launches per phase: 1 TMA pipeline, 0 direct 32x8, 2 direct 8x4
+                              (cooperative launches have their own, mgpu_set_engine) */
     int pad_;
     double autotune_us[3]; /* plain_path -1: measured microseconds per coarse step of paths 0, 1, 2 (else 0) */
 } mgpu_info;
@@ -251,10 +252,15 @@ int mgpu_batch_set_stream(mgpu_batch *b, void *stream);
  * of the batch: blocks claim units of work in order and a stage of an image
  * (a phase of its coarse step, an interface wave) starts when its previous
  * stage is complete, as device-side counters show; `group` images (0 = all)
- * are interleaved at a time.  Until this is called, a batch whose images are
- * small enough (state of up to twice the L2 each) steps groups of images in
- * cooperative launches of many coarse steps, as single contexts do
- * (mgpu_set_engine), others by engine 0.  All give bit-identical states. */
+ * are interleaved at a time.  Until this is called, groups of images (populations of
+ * up to three quarters of the L2 cache) are stepped by cooperative launches of many
+ * coarse steps, as single contexts are (mgpu_set_engine), and by engine 0 instead: calls
+ * of 1, 2, 4 or 6 steps of up to 12 levels in all (2 steps where every image has one
+ * level; 1 where there are several groups), batches that hold both images with
+ * populations beyond the L2 and smaller ones, images that do not fit the kernel's tables,
+ * and streams of fewer SMs than the device has.  How the contexts step on their own
+ * (plain_path, concurrent, mgpu_set_engine) does not matter to a batch, but that engine
+ * 0 takes the plain-cell kernel of each.  All give bit-identical states. */
 #define MGPU_ENGINE_STREAMS 0
 #define MGPU_ENGINE_PERSISTENT 1
 int mgpu_batch_set_engine(mgpu_batch *b, int engine, int group);

@@ -1692,7 +1692,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ads_persistent(const __grid_cons
 // memory.  A cell's populations are then the only round trip to memory.
 //
 // Measured on a GB300, us per coarse step without / with residuals: single block
-// 64^2 3.6 / 4.4, 128^2 3.7 / 4.5, 512^2 5.3 / 7.1, 1024^2 12.1 / 15.5, two levels
+// 64^2 3.6 / 4.4, 128^2 3.7 / 4.5, 512^2 5.3 / 7.1, 1024^2 11.7 / 15.7, two levels
 // 256^2 16.1 / 17.6, 1024^2 34 / 37; the launches per phase 6.1 / 10.7, 6.2 / 10.4,
 // 9.3 / 17.4, 16.4 / 34.7, 22.9 / 27.5, 42.8 / 55.9.  A grid barrier takes 0.85 us,
 // a warp of special cells about 2.5: what small images wait for.  At 1024^2 the

@@ -2919,6 +2919,13 @@ void batch_leave(mgpu_batch *b)
 // steps: 235, launches 238), and an odd number of steps leaves the graph's parity.
 bool batch_coop(mgpu_batch *b, int n_steps)
 {
+    size_t levels = 0, large = 0;
+    for (auto *c : b->ctxs)
+    {
+        levels += c->lv.size();
+        large += c->populations > c->l2 ? 1 : 0;
+    }
+    if (large > 0 && large < b->ctxs.size()) return false;
     if (b->coop.empty())
     {
         if (is_capturing(b->stream)) return false; // nothing is allocated during a capture
@@ -2931,14 +2938,8 @@ bool batch_coop(mgpu_batch *b, int n_steps)
     }
     for (auto &g : b->coop)
         if (!g->ok || g->grid > b->stream_sms) return false;
-    size_t levels = 0, large = 0;
-    for (auto *c : b->ctxs)
-    {
-        levels += c->lv.size();
-        large += c->populations > c->l2 ? 1 : 0;
-    }
-    if (large > 0 && large < b->ctxs.size()) return false;
-    const bool few = n_steps < (levels == b->ctxs.size() ? 4 : 8) && (n_steps % 2 == 0 || (n_steps == 1 && b->coop.size() > 1));
+    const bool few = n_steps < (levels == b->ctxs.size() ? 4 : 8) &&
+                     (n_steps % 2 == 0 || (n_steps == 1 && b->coop.size() > 1));
     return !(few && levels <= 12);
 }
 
