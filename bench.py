@@ -759,9 +759,10 @@ def main():
                        "levels": [int(im["levels"]) for im in imgs] if args.workload == "config4" else imgs[0]["levels"],
                        "lu_per_step_per_gpu": lu_step, "device_state_mb_per_gpu": round(state_mb, 1),
                        "l2": "inputs larger than L2 (state of the batch > 129 MB)" +
-                             ("; a cooperative launch steps one L2-sized group of images up to 500 times"
+                             ("; a cooperative launch steps one group of images (3/4 of the L2) up to 500 times"
                               if args.engine < 0 else ""),
-                       "graph": {-1: "cooperative launches of up to 500 coarse steps per group of images",
+                       "graph": {-1: "cooperative launches of up to 500 coarse steps per group of images (images beyond "
+                                     "the L2 beside smaller ones: as engine 0)",
                                  0: "one CUDA graph of 2 coarse steps for the whole batch, images on L2-sized "
                                     "concurrent streams",
                                  1: "one CUDA graph of 2 coarse steps for the whole batch, one persistent launch "
