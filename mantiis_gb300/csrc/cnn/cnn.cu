@@ -339,10 +339,16 @@ int tc_ntile(int pixel_ctas, int cout)
     return nt;
 }
 
+// SMs of the current device, asked for once per device
 int sm_count()
 {
+    static std::atomic<int> known[64];
     int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaGetDevice(&dev) != cudaSuccess) return sms;
+    std::atomic<int> *slot = dev < 64 ? &known[dev] : nullptr;
+    if (slot && slot->load(std::memory_order_relaxed)) return slot->load(std::memory_order_relaxed);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && slot)
+        slot->store(sms, std::memory_order_relaxed);
     return sms;
 }
 

@@ -134,16 +134,17 @@ class Conv3x3:
 
         n, _, h, w = x.shape
         shape = (n, self.cout, h, w)
-        if skip is not None and tuple(skip.shape) != shape:
-            raise ValueError(f"skip connection of shape {tuple(skip.shape)}, output {shape}")
-        new = lambda: torch.empty(shape, dtype=torch.float32, device="cuda")
-        if skip is not None and not TENSOR_CORES:
-            y, d = new() if keep else None, new()
-            _check(cnn_lib().cnn_conv3x3_forward_add(_ptr(x), _ptr(self.w16), _ptr(self.b), _ptr(y), _ptr(skip),
-                                                     _ptr(d), n, self.cin, self.cout, h, w, 1 if relu else 0,
-                                                     _stream()), "conv forward")
-            return y, d
-        y = new()
+        if skip is not None:
+            if tuple(skip.shape) != shape:
+                raise ValueError(f"skip connection of shape {tuple(skip.shape)}, output {shape}")
+            if not TENSOR_CORES:
+                y = torch.empty(shape, dtype=torch.float32, device="cuda") if keep else None
+                d = torch.empty(shape, dtype=torch.float32, device="cuda")
+                _check(cnn_lib().cnn_conv3x3_forward_add(_ptr(x), _ptr(self.w16), _ptr(self.b), _ptr(y), _ptr(skip),
+                                                         _ptr(d), n, self.cin, self.cout, h, w, 1 if relu else 0,
+                                                         _stream()), "conv forward")
+                return y, d
+        y = torch.empty(shape, dtype=torch.float32, device="cuda")
         fwd = cnn_lib().cnn_conv3x3_forward_tc if TENSOR_CORES else cnn_lib().cnn_conv3x3_forward
         _check(fwd(_ptr(x), _ptr(self.w16), _ptr(self.b), _ptr(y), n, self.cin, self.cout, h, w, 1 if relu else 0,
                    _stream()), "conv forward")
@@ -158,13 +159,13 @@ class Conv3x3:
         import torch
 
         n, _, h, w = x.shape
+        if relu is not None and need_dx and relu.shape != x.shape:
+            raise ValueError(f"ReLU output of shape {tuple(relu.shape)}, layer input {tuple(x.shape)}")
         L = cnn_lib()
         _check(L.cnn_conv3x3_backward_weight(_ptr(x), _ptr(dy), _ptr(self.dw), _ptr(self.db), n, self.cin, self.cout,
                                              h, w, _stream()), "conv weight gradient")
         if not need_dx:
             return None
-        if relu is not None and relu.shape != x.shape:
-            raise ValueError(f"ReLU output of shape {tuple(relu.shape)}, layer input {tuple(x.shape)}")
         if relu is not None and not TENSOR_CORES:
             dx, masked = torch.empty_like(x) if keep else None, torch.empty_like(x)
             _check(L.cnn_conv3x3_backward_data_relu(_ptr(dy), _ptr(self.w16), _ptr(dx), _ptr(relu), _ptr(masked), n,
